@@ -238,6 +238,16 @@ static int create_sector(const edg_model* m, int n_ones, int kx, int ky, int kz,
       group_ch[g].push_back(c);
     }
   }
+  // distinct diagonal parts: a row's Ezz counts its anti-aligned pairs of each
+  {
+    std::vector<double> facs;
+    for (TermGroup& g : groups) {
+      g.fid = (int)(std::find(facs.begin(), facs.end(), g.fac) - facs.begin());
+      if (g.fid == (int)facs.size()) facs.push_back(g.fac);
+    }
+    P.n_facs = (int)facs.size();
+    for (int k = 0; k < P.n_facs && P.n_facs <= kMaxFacs; ++k) P.facs[k] = facs[k];
+  }
   std::vector<ChTerm> ch;
   for (size_t g = 0; g < groups.size(); ++g) {
     groups[g].ch_begin = (int)ch.size();

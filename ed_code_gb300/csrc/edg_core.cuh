@@ -38,6 +38,7 @@ constexpr int kMaxGroups = 512;    // distinct flipped pairs
 constexpr int kMaxChTerms = 1024;  // chirality terms
 constexpr int kMaxBowties = 65536;
 constexpr int kRecBits = 96;       // Lin indices per rank record
+constexpr int kMaxFacs = 4;        // distinct diagonal parts counted per row (FP64 sums beyond that)
 constexpr int kMaxTorusRow = 10;   // row-rotation search tables hold 2^Lx entries
 
 EDG_HD int popc64(uint64_t x) {
@@ -76,6 +77,8 @@ struct TermGroup {
   uint64_t mask;
   int a, b;
   int ch_begin, ch_end;
+  int fid;              // index of fac among SectorParams::facs (when n_facs <= kMaxFacs)
+  int pad;
   double fac;           // sum over bonds of 0.25*lambda*J (diagonal part)
   double Bre[2], Bim[2];
 };
@@ -121,6 +124,10 @@ struct SectorParams {
   uint8_t g2cls[64];
   int n_cls, pad2;
   int64_t n_targets;
+  // Distinct values of TermGroup::fac (one per coupling strength); n_facs >
+  // kMaxFacs: facs is not filled and rows sum fac itself.
+  int n_facs, pad3;
+  double facs[kMaxFacs];
 };
 
 // --------------------------------------------------------------------------
@@ -307,6 +314,82 @@ EDG_HD Orbit orbit_torus(uint64_t t, const SectorParams& P, const uint8_t* nk, c
   }
   return o;
 }
+
+// ---- the same search on packed rows (Lx <= 8, Ly <= 8) --------------------
+// The rotation minima of all rows sit in one word, row y in byte y and 0xFF
+// above row Ly - 1, so a flip that touches two rows changes two bytes and the
+// smallest minimum and the rows that reach it come from a few byte-parallel
+// operations, the same for every lane of a warp whatever rows its states have.
+// States are 32-bit words when N <= 32, and so are the packed minima when
+// Ly <= 4: 64-bit shifts and masks cost two to four instructions each.
+#if defined(__CUDACC__)
+template <typename St, typename Kb>
+struct PackedRows {
+  using State = St;  // uint32_t (N <= 32) or uint64_t
+  using Bytes = Kb;  // uint32_t (Ly <= 4) or uint64_t
+
+  static __device__ __forceinline__ Bytes set(Bytes kb, int at, int v) {  // byte at bit offset `at`
+    return (kb & ~((Bytes)0xFF << at)) | ((Bytes)v << at);
+  }
+  static __device__ __forceinline__ Bytes pack(State t, const SectorParams& P, const uint8_t* nk) {
+    const State rmask = ((State)1 << P.L1) - 1;
+    Bytes kb = ~(Bytes)0;
+    for (int y = 0; y < P.L2; ++y) kb = set(kb, 8 * y, nk[(int)((t >> (P.L1 * y)) & rmask)]);
+    return kb;
+  }
+  static __device__ __forceinline__ Bytes valid(const SectorParams& P) {  // 0x80 in the rows there are
+    return (Bytes)(0x8080808080808080ull >> (8 * (8 - P.L2)));
+  }
+  static __device__ __forceinline__ uint32_t equal32(uint32_t kb, uint32_t mm) {  // 0x80 where the bytes agree
+    const uint32_t x = kb ^ mm;
+    return ~(((x & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | x) & 0x80808080u;
+  }
+  static __device__ __forceinline__ uint32_t min32(uint32_t kb) {  // byte minima of the even and odd bytes
+    return __vminu2(kb & 0x00FF00FFu, (kb >> 8) & 0x00FF00FFu);
+  }
+  // smallest byte of kb; hit: 0x80 in every valid row's byte that equals it
+  static __device__ __forceinline__ int min_rows(Bytes kb, Bytes valid, Bytes& hit) {
+    uint32_t m2 = min32((uint32_t)kb);
+    if (sizeof(Bytes) == 8) m2 = __vminu2(m2, min32((uint32_t)((uint64_t)kb >> 32)));
+    const uint32_t m = min(m2 & 0xFFFFu, m2 >> 16);
+    const uint32_t mm = m * 0x01010101u;
+    Bytes z = equal32((uint32_t)kb, mm);
+    if (sizeof(Bytes) == 8) z |= (Bytes)((uint64_t)equal32((uint32_t)((uint64_t)kb >> 32), mm) << 32);
+    hit = z & valid;
+    return (int)m;
+  }
+  static __device__ __forceinline__ bool single(Bytes hit) { return (hit & (hit - 1)) == 0; }
+  static __device__ __forceinline__ int row_of(Bytes hit) {  // lowest row in hit
+    return (sizeof(Bytes) == 8 ? __ffsll((long long)hit) : __ffs((int)hit)) / 8 - 1;
+  }
+  static __device__ __forceinline__ Orbit search(State t, Bytes hit, const SectorParams& P, const uint16_t* rots) {
+    const int Lx = P.L1, Ly = P.L2, N = P.n_sites;
+    const State rmask = ((State)1 << Lx) - 1, full = (State)P.full_mask;
+    State best = ~(State)0;
+    int g = 0, stab = 0;
+    while (hit) {
+      const int y = row_of(hit);
+      hit &= hit - 1;
+      const int b = Ly - 1 - y;
+      uint32_t rs = rots[(int)((t >> (Lx * y)) & rmask)];
+      const State u = b == 0 ? t : ((t << (Lx * b)) | (t >> (N - Lx * b))) & full;
+      while (rs) {
+        const int a = __ffs((int)rs) - 1;
+        rs &= rs - 1;
+        const State v = a == 0 ? u : ((u << a) & (State)P.rot_hi[a]) | ((u >> (Lx - a)) & (State)P.rot_lo[a]);
+        if (v < best || stab == 0) {
+          best = v;
+          g = a + Lx * b;
+          stab = 1;
+        } else if (v == best) {
+          ++stab;
+        }
+      }
+    }
+    return Orbit{(uint64_t)best, g, stab};
+  }
+};
+#endif
 
 // Is t an allowed representative (rep == t and p_id, Momentum_Basis.cpp:538-540
 // and :761-770)?  Returns its stabiliser count, or 0.

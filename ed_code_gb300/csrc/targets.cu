@@ -42,121 +42,226 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 constexpr int kTgtThreads = 32 * kWarpsPerBlock;
+constexpr int kPassThreads = 128;
 constexpr int kMaxChPerGroup = 4;
 
-// anti-aligned groups of state s, 32 at a time: bit l of word r is group 32r+l
-template <int NW>
-__device__ __forceinline__ void anti_words(uint64_t s, const HvSmem<double>& H, int ng, uint32_t (&words)[NW],
-                                           double& fac_lane) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int r = 0; r < NW; ++r) {
-    const int g = 32 * r + lane;
-    bool a = false;
-    if (g < ng) {
-      a = popc64(s & H.groups[g].mask) == 1;
-      if (a) fac_lane += H.groups[g].fac;
+// A flip group as the passes below stage it: what a row needs to find out
+// whether the pair is anti-aligned, and where its sites sit on a packed torus.
+struct PassGroup {
+  uint64_t mask;
+  uint64_t facadd;        // 1 << 16 * fid: counts the row's anti-aligned pairs by diagonal part
+  double fac;
+  uint16_t off;           // first value variant
+  int16_t a, ch_begin, ch_end;
+  int8_t sa, sb, ba, bb;  // packed torus: bit offset of each site's row in the state, of its byte
+  int8_t top, pad[3];     // packed torus: the pair touches the top row
+};
+
+// Which orbit search the passes use: the reference's walk, the row-rotation
+// search, or the row-rotation search on packed rows (row length and row count
+// up to 8) with 32-bit states and minima, 32-bit states, or 64-bit ones.
+constexpr int kOrbWalk = 0, kOrbTorus = 1, kOrbPacked = 2, kOrbPacked32 = 3, kOrbPacked64 = 4;
+template <int kOrb>
+struct OrbRows {
+  using T = PackedRows<uint64_t, uint64_t>;
+};
+template <>
+struct OrbRows<kOrbPacked> {
+  using T = PackedRows<uint32_t, uint32_t>;
+};
+template <>
+struct OrbRows<kOrbPacked32> {
+  using T = PackedRows<uint32_t, uint64_t>;
+};
+int orb_of(const SectorParams& P) {
+  if (!P.torus) return kOrbWalk;
+  if (P.L1 > 8 || P.L2 > 8) return kOrbTorus;
+  return P.n_sites > 32 ? kOrbPacked64 : P.L2 <= 4 ? kOrbPacked : kOrbPacked32;
+}
+
+struct PassSmem {
+  PassGroup* groups;
+  int8_t* z;  // chirality sites
+  const uint8_t* nk;
+  const uint16_t* rots;
+  const uint64_t *p1, *p2, *p3;
+};
+
+size_t pass_smem_bytes(const SectorParams& P, int orb, int row_bits, int n_chunks, int n_perm) {
+  size_t b = align16(sizeof(PassGroup) * P.n_groups) + align16(P.n_ch);
+  if (orb == kOrbWalk) return b + (size_t)n_perm * n_chunks * 256 * sizeof(uint64_t);
+  return b + align16((size_t)3 << row_bits);
+}
+
+template <int kOrb>
+__device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, const uint16_t* voff,
+                               const uint16_t* order, uint8_t* sm) {
+  PassSmem H{};
+  size_t off = 0;
+  H.groups = reinterpret_cast<PassGroup*>(sm);
+  off += align16(sizeof(PassGroup) * P.n_groups);
+  H.z = reinterpret_cast<int8_t*>(sm + off);
+  off += align16(P.n_ch);
+  for (int at = threadIdx.x; at < P.n_groups; at += blockDim.x) {
+    const int g = order[at];
+    const TermGroup src = V.groups[g];
+    PassGroup d{};
+    d.mask = src.mask;
+    d.facadd = P.n_facs <= kMaxFacs ? 1ull << (16 * src.fid) : 0;
+    d.fac = src.fac;
+    d.off = voff[g];
+    d.a = (int16_t)src.a;
+    d.ch_begin = (int16_t)src.ch_begin;
+    d.ch_end = (int16_t)src.ch_end;
+    if (kOrb >= kOrbPacked) {
+      const int ya = src.a / P.L1, yb = src.b / P.L1;
+      d.sa = (int8_t)(P.L1 * ya);
+      d.sb = (int8_t)(P.L1 * yb);
+      d.ba = (int8_t)(8 * ya);
+      d.bb = (int8_t)(8 * yb);
+      d.top = ya == P.L2 - 1 || yb == P.L2 - 1;
     }
-    words[r] = __ballot_sync(0xffffffffu, a);
+    H.groups[at] = d;
   }
-}
-
-// group of the k-th anti-aligned pair
-template <int NW>
-__device__ __forceinline__ int select_group(const uint32_t (&words)[NW], int k) {
-  uint32_t wsel = 0;
-  int qsel = 0, before = 0, acc = 0;
-#pragma unroll
-  for (int q = 0; q < NW; ++q) {
-    const int c = __popc(words[q]);
-    if (k >= acc && k < acc + c) {
-      wsel = words[q];
-      qsel = q;
-      before = acc;
+  for (int m = threadIdx.x; m < P.n_ch; m += blockDim.x) H.z[m] = (int8_t)V.ch[m].z;
+  if (kOrb == kOrbWalk) {
+    const int n = V.n_perm * V.n_chunks * 256;
+    uint64_t* p = reinterpret_cast<uint64_t*>(sm + off);
+    for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = V.perms[i];
+    H.p1 = p;
+    H.p2 = p + V.n_chunks * 256;
+    H.p3 = p + 2 * V.n_chunks * 256;
+  } else {
+    const int n = 1 << V.row_bits;
+    uint16_t* rots = reinterpret_cast<uint16_t*>(sm + off);
+    uint8_t* nk = sm + off + 2 * n;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      rots[i] = V.rots[i];
+      nk[i] = V.nk[i];
     }
-    acc += c;
+    H.rots = rots;
+    H.nk = nk;
   }
-  return 32 * qsel + (int)__fns(wsel, 0u, k - before + 1);
+  return H;
 }
 
-template <int NW>
-__device__ __forceinline__ int total(const uint32_t (&words)[NW]) {
-  int n = 0;
-#pragma unroll
-  for (int q = 0; q < NW; ++q) n += __popc(words[q]);
-  return n;
-}
-
-// Pass 1 (count) and pass 2 (fill) share this walk over a row's targets: one
-// warp per row, lane k resolves the row's k-th anti-aligned pair.
-// The fill pass writes each entry's value id as remap[(pair variant) x class],
-// the index into the deduplicated value table, packed above the column when
-// cb > 0 (csr_row.cuh).
-template <bool kTorus, int NW, bool kFill>
-__global__ void __launch_bounds__(kTgtThreads) k_tgt_pass(SectorView V, const uint16_t* __restrict__ voff,
-                                                          const uint16_t* __restrict__ remap, int cb,
-                                                          uint32_t* __restrict__ counts, double* __restrict__ ezz,
-                                                          const uint64_t* __restrict__ row_ptr,
-                                                          uint32_t* __restrict__ col, uint16_t* __restrict__ vid) {
+// Pass 1 (count) and pass 2 (fill) share this walk over the rows' targets: a
+// thread owns a row and all of them go through the flip groups together, those
+// of high sites first (`order`).
+// Neighbouring rows are neighbouring representatives, equal in their high
+// sites: a group of high sites is anti-aligned in the whole warp or in none of
+// it (and is then skipped by the warp), its search takes the same turns in
+// every lane, and its rank records and remap entries come from neighbouring
+// addresses.  Counting needs no rank for a target that is alone in its orbit
+// search (one candidate translate): its stabiliser is trivial, so it is
+// allowed.  The fill pass writes each entry's value id as
+// remap[(pair variant) x class], the index into the deduplicated value table,
+// packed above the column when cb > 0 (csr_row.cuh).
+//
+// Both passes are bound by integer issue (ALU pipe 65 %, 17-20 lanes of a warp
+// active), not by memory.  With a warp per row and a lane per pair they took
+// 18.7 + 22.8 ms on the 18.8-million-state 8x4 triangular sector; this form
+// took 7.9 + 14.1 ms with 64-bit states, and the sector up to its first H v
+// 54 ms, 34 ms, and 29 ms with 32-bit states.
+template <int kOrb, bool kFill>
+__global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const uint16_t* __restrict__ voff,
+                                                           const uint16_t* __restrict__ order,
+                                                           const uint16_t* __restrict__ remap, int cb,
+                                                           uint32_t* __restrict__ counts, double* __restrict__ ezz,
+                                                           const uint64_t* __restrict__ row_ptr,
+                                                           uint32_t* __restrict__ col, uint16_t* __restrict__ vid) {
   __shared__ SectorParams P;
-  __shared__ uint16_t off[kMaxGroups];
   extern __shared__ __align__(16) uint8_t sm[];
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
     reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
   __syncthreads();
-  for (int g = threadIdx.x; g < P.n_groups; g += blockDim.x) off[g] = voff[g];
-  const HvSmem<double> H = stage_hv<double, kTorus>(V, P, sm);
+  const PassSmem H = stage_pass<kOrb>(V, P, voff, order, sm);
   __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const uint32_t lt = (1u << lane) - 1u;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  for (int64_t i = warp; i < P.n_p; i += n_warps) {
-    const uint64_t s = V.reps[i];
-    uint32_t words[NW];
-    double fac = 0.0;
-    anti_words<NW>(s, H, P.n_groups, words, fac);
-    const int nt = total(words);
-    uint64_t pos = kFill ? row_ptr[i] : 0;
+  using R = typename OrbRows<kOrb>::T;
+  using St = typename R::State;
+  using Kb = typename R::Bytes;
+  const int ng = P.n_groups, Lx = P.L1;
+  const St rmask = ((St)1 << Lx) - 1;
+  const Kb valid = kOrb >= kOrbPacked ? R::valid(P) : 0;
+  const bool count_facs = P.n_facs <= kMaxFacs;
+  const int64_t n_p = P.n_p, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_p; base += stride) {
+    const int64_t i = base + threadIdx.x;
+    const bool live = i < n_p;
+    const St s = live ? (St)V.reps[i] : 0;  // no pair is anti-aligned past the end
+    Kb kb = 0;
+    uint64_t facs = 0, pos = 0;
+    int mstar = 0;
+    bool uniq = false;
     uint32_t cnt = 0;
-    for (int k0 = 0; k0 < nt; k0 += 32) {
-      const int k = k0 + lane;
-      bool ok = false;
-      uint32_t j = 0;
-      uint16_t id = 0;
-      if (k < nt) {
-        const int g = select_group(words, k);
-        const SmemGroup<double>& gr = H.groups[g];
-        Orbit o;
-        const int64_t jj = locate<double, kTorus>(s ^ gr.mask, V, P, H, o);
-        if (jj >= 0) {
-          ok = true;
-          j = (uint32_t)jj;
-          int variant = (int)((s >> gr.a) & 1u);
-          for (int m = gr.ch_begin, b = 1; m < gr.ch_end; ++m, ++b) variant |= (int)((s >> H.ch[m].z) & 1u) << b;
-          if (kFill) id = __ldg(remap + (off[g] + variant) * P.n_cls + P.g2cls[o.g]);
-        }
-      }
-      const uint32_t bal = __ballot_sync(0xffffffffu, ok);
-      if (kFill && ok) {
-        const uint64_t t = pos + __popc(bal & lt);
-        if (cb) {
-          col[t] = j | ((uint32_t)id << cb);
-        } else {
-          col[t] = j;
-          vid[t] = id;
-        }
-      }
-      pos += __popc(bal);
-      cnt += __popc(bal);
+    double fac = 0.0;
+    if (kFill && live) pos = row_ptr[i];
+    if (kOrb >= kOrbPacked) {
+      // s is a representative: its top row is at its rotation minimum and no
+      // row has a smaller one.  When it is the only row that reaches it and is
+      // aperiodic, a flip that leaves it alone and gives no other row a
+      // minimum <= mstar is its own representative with stabiliser 1.
+      kb = R::pack(s, P, H.nk);
+      Kb hit;
+      mstar = R::min_rows(kb, valid, hit);
+      uniq = R::single(hit) && H.rots[(int)((s >> (Lx * (P.L2 - 1))) & rmask)] == 1u;
     }
-    if (!kFill) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) fac += __shfl_down_sync(0xffffffffu, fac, o);
-      if (lane == 0) {
-        counts[i] = cnt;
-        ezz[i] = P.total_fac - 2.0 * fac;  // Ezz = sum_bonds lJ/4 - 2 sum_anti lJ/4
+    for (int g = 0; g < ng; ++g) {
+      const PassGroup& gr = H.groups[g];
+      const St pm = (St)gr.mask, both = s & pm;
+      const bool anti = both != 0 && both != pm;
+      if (!__any_sync(0xffffffffu, anti)) continue;
+      if (!anti) continue;
+      if (!kFill) {
+        facs += gr.facadd;
+        if (!count_facs) fac += gr.fac;
       }
+      const St t = s ^ pm;
+      Orbit o;
+      bool known = false;  // allowed for certain (counting)
+      if (kOrb >= kOrbPacked) {
+        const int na = H.nk[(int)((t >> gr.sa) & rmask)], nb = H.nk[(int)((t >> gr.sb) & rmask)];
+        if (uniq && !gr.top && na > mstar && nb > mstar) {
+          o = Orbit{(uint64_t)t, 0, 1};
+          known = true;
+        } else {
+          Kb hit;
+          R::min_rows(R::set(R::set(kb, gr.ba, na), gr.bb, nb), valid, hit);
+          if (!kFill && R::single(hit)) {
+            const uint32_t rs = H.rots[(int)((t >> (Lx * R::row_of(hit))) & rmask)];
+            known = (rs & (rs - 1)) == 0;
+          }
+          if (kFill || !known) o = R::search(t, hit, P, H.rots);
+        }
+      } else if (kOrb == kOrbTorus) {
+        o = orbit_torus(t, P, H.nk, H.rots);
+      } else {
+        o = orbit_walk(t, P, H.p1, H.p2, H.p3, V.n_chunks);
+      }
+      if (!kFill) {
+        if (known || position(o, V, P) >= 0) ++cnt;
+      } else {
+        const int64_t j = position(o, V, P);
+        if (j >= 0) {
+          int variant = (int)((s >> gr.a) & 1u);
+          for (int m = gr.ch_begin, b = 1; m < gr.ch_end; ++m, ++b) variant |= (int)((s >> H.z[m]) & 1u) << b;
+          const uint32_t id = __ldg(remap + (gr.off + variant) * P.n_cls + P.g2cls[o.g]);
+          if (cb) {
+            col[pos] = (uint32_t)j | (id << cb);
+          } else {
+            col[pos] = (uint32_t)j;
+            vid[pos] = (uint16_t)id;
+          }
+          ++pos;
+        }
+      }
+    }
+    if (!kFill && live) {
+      if (count_facs) {
+        for (int k = 0; k < P.n_facs; ++k) fac += P.facs[k] * (double)((facs >> (16 * k)) & 0xFFFFu);
+      }
+      counts[i] = cnt;
+      ezz[i] = P.total_fac - 2.0 * fac;  // Ezz = sum_bonds lJ/4 - 2 sum_anti lJ/4
     }
   }
 }
@@ -388,8 +493,6 @@ __global__ void __launch_bounds__(kTgtThreads) k_hv_csr(const uint64_t* __restri
   }
 }
 
-int n_words(int n_groups) { return n_groups <= 128 ? 4 : 8; }
-
 // Grid of a grid-stride kernel: the CTAs that fit on every SM at once, at most
 // cap per SM when cap > 0, no more than the work needs.
 template <typename K>
@@ -604,10 +707,23 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   S.pack_cb = (!want_split && vb < 32 && P.n_p < (int64_t(1) << cb)) ? cb : 0;
   const double entry_bytes = S.pack_cb ? 4.0 : 6.0;
 
+  // The passes take the groups of high sites first: consecutive representatives
+  // differ in their low sites, so a pair of high sites is anti-aligned in all
+  // rows of a warp or in none, and its targets in neighbouring rows are
+  // neighbours.
+  {
+    std::vector<uint16_t> order(P.n_groups);
+    for (int g = 0; g < P.n_groups; ++g) order[g] = (uint16_t)g;
+    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+      return groups[p].a != groups[q].a ? groups[p].a > groups[q].a : groups[p].b > groups[q].b;
+    });
+    voff.insert(voff.end(), order.begin(), order.end());
+  }
+
   cudaStream_t st = S.stream;
   const int64_t n = P.n_p;
   uint32_t* counts = nullptr;
-  uint16_t *d_voff = nullptr, *d_remap = nullptr;
+  uint16_t *d_voff = nullptr, *d_remap = nullptr;  // voff, then the groups' order
   unsigned long long *sums = nullptr, *tot = nullptr;
   const int64_t n_chunks = (n + kChunk - 1) / kChunk;
   cudaError_t e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
@@ -639,20 +755,17 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     err = "stored targets: out of device memory for the row data";
     return EDG_ERR_NOMEM;
   }
-  const bool torus = P.torus != 0;
-  const size_t smem = hv_smem_bytes<double>(P.n_groups, P.n_ch, torus, S.V.row_bits, S.V.n_chunks, S.V.n_perm);
-  const int nw = n_words(P.n_groups);
-  auto pass = [&](auto kern, bool fill) {
-    kern<<<grid_for(kern, smem, n * 32, kTgtThreads), kTgtThreads, smem, st>>>(
-        S.V, d_voff, d_remap, S.pack_cb, counts, S.ezz, S.row_ptr, fill ? S.col : nullptr, fill ? S.vid : nullptr);
+  const int orb = orb_of(P);
+  const size_t smem = pass_smem_bytes(P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm);
+  auto pass = [&](auto kern) {
+    kern<<<grid_for(kern, smem, n, kPassThreads), kPassThreads, smem, st>>>(
+        S.V, d_voff, d_voff + P.n_groups, d_remap, S.pack_cb, counts, S.ezz, S.row_ptr, S.col, S.vid);
   };
-  if (torus) {
-    if (nw == 4) pass(k_tgt_pass<true, 4, false>, false);
-    else pass(k_tgt_pass<true, 8, false>, false);
-  } else {
-    if (nw == 4) pass(k_tgt_pass<false, 4, false>, false);
-    else pass(k_tgt_pass<false, 8, false>, false);
-  }
+  if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, false>);
+  else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, false>);
+  else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, false>);
+  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, false>);
+  else pass(k_tgt_pass<kOrbWalk, false>);
   k_scan64_chunks<<<(unsigned)n_chunks, kScan, 0, st>>>(counts, n, sums);
   k_scan64_sums<<<1, kScan, 0, st>>>(sums, n_chunks, tot);
   k_scan64_apply<<<(unsigned)n_chunks, kScan, 0, st>>>(counts, n, sums, tot, S.row_ptr);
@@ -679,13 +792,11 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     return EDG_ERR_NOMEM;
   }
   S.ubuf.bytes = (size_t)(16 * n);
-  if (torus) {
-    if (nw == 4) pass(k_tgt_pass<true, 4, true>, true);
-    else pass(k_tgt_pass<true, 8, true>, true);
-  } else {
-    if (nw == 4) pass(k_tgt_pass<false, 4, true>, true);
-    else pass(k_tgt_pass<false, 8, true>, true);
-  }
+  if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, true>);
+  else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, true>);
+  else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, true>);
+  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, true>);
+  else pass(k_tgt_pass<kOrbWalk, true>);
   e = cudaStreamSynchronize(st);
   cleanup();
   if (e != cudaSuccess) {

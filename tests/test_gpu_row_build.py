@@ -1,0 +1,37 @@
+"""Stored rows built by each orbit search, at the edges of their ranges.
+
+The passes that search the targets take 32- or 64-bit states and 4 or 8 packed
+row minima by the torus (N <= 32, Ly <= 4; N <= 32; else), the general
+row-rotation search for rows longer than 8 sites, and the reference's walk
+elsewhere.  Each is compared with the oracle's sHv on a sector of few flipped
+spins, at the tolerance of the other FP64 parity tests.
+"""
+import numpy as np
+import pytest
+
+import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("Lx,Ly,Sz,k,J2", [
+    (4, 4, 1, (1, 3), 0.0),     # 32-bit states, 4 rows
+    (8, 4, 11, (5, 2), 0.0),    # N = 32: the largest 32-bit state, rows of 8
+    (4, 8, 11, (1, 6), 0.0),    # 8 rows: the largest packed word
+    (6, 5, 10, (2, 3), 0.4),    # 32-bit states, more than 4 rows, two couplings
+    (8, 5, -16, (7, 4), 0.0),   # N = 40: 64-bit states
+    (9, 4, -14, (4, 1), 0.0),   # rows longer than 8: the general search
+])
+def test_stored_rows_of_every_search_match_oracle(cuda_device, Lx, Ly, Sz, k, J2):
+    from ed_code_gb300 import lattice as L
+    from ed_code_gb300 import sector
+
+    model = L.make_model(L.TorusSpec("triangular", Lx, Ly, Jz=0.7, J2=J2, Ch=0.3), Sz, *k, bowties=False)
+    ref = O.OracleSector(model)
+    sec = sector.GpuSector(model)
+    assert sec.n_p == ref.n_p
+    v = O.splitmix_vector(sec.n_p, 5)
+    w = ref.hv(v)
+    assert sec.build_targets()
+    assert sec.info["n_targets"] == sec.count_offdiag()
+    assert np.abs(sec.sHv(v) - w).max() / max(1.0, np.abs(w).max()) <= 1e-13
