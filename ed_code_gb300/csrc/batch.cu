@@ -12,7 +12,7 @@
 // reads its segment's descriptor.  One step is nine kernels:
 //
 //   k_b_hv          u_j = V_j / norm was written by the previous step;
-//                   w = H V_j (CSR rows, lanes_per_row lanes per row) and the
+//                   w = H V_j (lanes_per_row / 2 entries of a row in flight) and the
 //                   tile's partial of alpha_j = Re<V_j|w>
 //   k_b_step        w -= alpha_j V_j + beta_j V_{j-1} and the tile's |w|^2
 //   k_b_cgs_dot     classical Gram-Schmidt: the tile's <V_k|w>, k <= j
@@ -171,77 +171,36 @@ __device__ __forceinline__ void seg_sum(const double* part, int k0, int k1, doub
 // ticket counters of a segment, one per fused reduction
 enum { kCntAlpha = 0, kCntNorm = 1, kCntDecide = 2, kCntBeta = 3, kCntAdvance = 4, kCnts = 8 };
 
-// w = H V_j on the tile's rows: 32/LPR rows per warp, LPR lanes per row, each
-// row summed by the single-sector kernel's routines (unrolled entry loads,
-// streaming hint on the row data, L2 evict_last on u).  Pipelined like the
-// single-sector kernel: a warp loads the head entries of its next rows (and
-// the offsets of the rows after) before it gathers for the current ones.
-//
-// Then alpha_j = Re<V_j|w>: the tile's partial (exact products summed in
-// float-float per thread, FP64 across the CTA), closed per segment by the
-// last CTA.
-template <int LPR>
+// w = H V_j on the tile's rows, a warp per slice of 32 rows (csr_row.cuh), and
+// the tile's partial of alpha_j = Re<V_j|w> (exact products summed in
+// float-float per thread, FP64 across the CTA), closed per segment by the last
+// CTA.  kU: entries of a row in flight.
+template <int kU>
 __global__ void __launch_bounds__(kThreads) k_b_hv(const SegDev* __restrict__ segs, const SegState* __restrict__ ss,
                                                    const TileDev* __restrict__ tiles, const int* __restrict__ tb,
                                                    double* __restrict__ part, int* __restrict__ cnt) {
   const TileDev t = tiles[blockIdx.x];
   if (ss[t.seg].status != kRunning) return;
   const SegDev& S = segs[t.seg];
-  constexpr int kRowsPerWarp = 32 / LPR;
-  constexpr int kU = head_entries<LPR>();
-  const int lane = threadIdx.x & 31, sl = lane % LPR, sub = lane / LPR, wid = threadIdx.x >> 5;
   const float2* v = S.V + (int64_t)ss[t.seg].j * S.n;
-  const int rows_per_pass = (kThreads / 32) * kRowsPerWarp;
   const uint64_t pl = l2_evict_last();
-  auto offsets = [&](int r, uint64_t& b, uint64_t& e) {
-    b = e = 0;
-    if (r < t.rows) {
-      b = S.row_ptr[t.row0 + r];
-      e = S.row_ptr[t.row0 + r + 1];
-    }
-  };
-  int r = wid * kRowsPerWarp + sub;
-  uint64_t beg, end, beg1, end1;
-  offsets(r, beg, end);
-  offsets(r + rows_per_pass, beg1, end1);
-  uint32_t e[kU];
-  uint16_t h[kU];
-  csr_head<LPR, kByVid, 1>(beg, end, sl, S.col, S.vid, 0, e, h);
-  for (int r0 = 0; r0 < t.rows; r0 += rows_per_pass) {
-    uint64_t beg2, end2;
-    offsets(r + 2 * rows_per_pass, beg2, end2);
-    uint32_t en[kU];
-    uint16_t hn[kU];
-    csr_head<LPR, kByVid, 1>(beg1, end1, sl, S.col, S.vid, 0, en, hn);
-    float ar, ai;
-    csr_finish<float, LPR, false, 1, kByVid>(beg, end, sl, S.col, S.vid, S.pack_cb, S.vtab, S.u, 0, pl, e, h, ar,
-                                             ai);
-    if (r < t.rows && sl == 0) {
-      const int64_t i = t.row0 + r;
-      const float ni = (float)S.nrm[S.lid[i]];
-      const float d = (float)S.ezz[i];
-      S.w[i] = row_out(ar, ai, ni, d, v[i]);
-    }
-    r += rows_per_pass;
-    beg = beg1;
-    end = end1;
-    beg1 = beg2;
-    end1 = end2;
-#pragma unroll
-    for (int q = 0; q < kU; ++q) {
-      e[q] = en[q];
-      h[q] = hn[q];
-    }
-  }
-  __syncthreads();  // the tile's w rows are written
+  const RowsView<float> R{S.row_ptr, S.col, S.vid, S.vtab, S.u, S.pack_cb};
   FFAcc sr, si;
-  for (int rr = threadIdx.x; rr < t.rows; rr += blockDim.x) {
-    const int64_t i = t.row0 + rr;
-    const float2 y = S.w[i], x = v[i];
-    sr.add_prod(x.x, y.x);
-    sr.add_prod(x.y, y.y);
-    si.add_prod(x.x, y.y);
-    si.sub_prod(x.y, y.x);
+  for (int r0 = 0; r0 < t.rows; r0 += kThreads) {  // the tile starts at a multiple of 32
+    const int r = r0 + threadIdx.x;
+    const int64_t i = t.row0 + r;
+    const Slice s = slice_at(R.row_ptr, i, t.row0 + t.rows);
+    float sum[2];
+    slice_sums<float, 1, kByVid, 1, kU, kU, true>(R, s, 0, s.mx, 0, pl, sum);
+    if (r < t.rows) {
+      const float2 x = v[i];
+      const float2 y = row_out(sum[0], sum[1], (float)S.nrm[S.lid[i]], (float)S.ezz[i], x);
+      S.w[i] = y;
+      sr.add_prod(x.x, y.x);
+      sr.add_prod(x.y, y.y);
+      si.add_prod(x.x, y.y);
+      si.sub_prod(x.y, y.x);
+    }
   }
   double a = sr.value(), b = si.value();
   block_sum2(a, b);
@@ -653,24 +612,20 @@ __global__ void __launch_bounds__(kThreads) k_f_u(const FinVec* __restrict__ vs,
 
 __global__ void __launch_bounds__(kThreads) k_f_hv(const FinVec* __restrict__ vs, const FinTile* __restrict__ ts,
                                                    double* __restrict__ part, int* __restrict__ cnt) {
-  constexpr int LPR = 8, kRows = 32 / LPR, kPass = (kThreads / 32) * kRows;
   const FinTile t = ts[blockIdx.x];
   const FinVec& V = vs[t.v];
-  const int lane = threadIdx.x & 31, sl = lane % LPR, sub = lane / LPR, wid = threadIdx.x >> 5;
+  const uint64_t pl = l2_evict_last();
+  const RowsView<double> R{V.row_ptr, V.col, V.vid, V.vtab, V.u, V.pack_cb};
   Acc s0, s1;
-  for (int base = wid * kRows; base < t.rows; base += kPass) {  // uniform within the warp
-    const int r = base + sub;
-    uint64_t beg = 0, end = 0;
+  for (int r0 = 0; r0 < t.rows; r0 += kThreads) {  // tiles start at multiples of 32 rows
+    const int r = r0 + threadIdx.x;
+    const int64_t i = t.row0 + r;
+    const Slice s = slice_at(R.row_ptr, i, t.row0 + t.rows);
+    double sum[2];
+    slice_sums<double, 1, kByVid, 1, 8, 8, false>(R, s, 0, s.mx, 0, pl, sum);
     if (r < t.rows) {
-      beg = V.row_ptr[t.row0 + r];
-      end = V.row_ptr[t.row0 + r + 1];
-    }
-    double ar, ai;
-    csr_row<double, LPR, false, 1, kByVid>(beg, end, sl, V.col, V.vid, V.pack_cb, V.vtab, V.u, ar, ai);
-    if (r < t.rows && sl == 0) {
-      const int64_t i = t.row0 + r;
       const double2 xi = V.x[i];
-      const double2 h = row_out(ar, ai, V.nrm[V.lid[i]], V.ezz[i], xi);
+      const double2 h = row_out(sum[0], sum[1], V.nrm[V.lid[i]], V.ezz[i], xi);
       V.hx[i] = h;
       s0.add(xi.x * xi.x + xi.y * xi.y);
       s1.add(xi.x * h.x + xi.y * h.y);
@@ -1178,9 +1133,9 @@ int rebuild(Batch& B) {
   // second-pass decision, subtraction; the second pass ends with beta);
   // V_{j+1}, u_{j+1}, the step counter and the convergence test
   int* cnt = B.d_cnt;
-  if (lpr == 8) k_b_hv<8><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
-  else if (lpr == 32) k_b_hv<32><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
-  else k_b_hv<16><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
+  if (lpr == 8) k_b_hv<4><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
+  else if (lpr == 32) k_b_hv<16><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
+  else k_b_hv<8><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
   k_b_step<<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
   for (int pass = 0; pass < 2; ++pass) {
     k_b_cgs_dot<<<dim3(nt, kCgsY), kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, nt, B.d_part, pass);

@@ -589,7 +589,7 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
   else if (wa.type == cudaMemoryTypeHost)
     w_dev = wa.devicePointer;
   if (e == cudaSuccess && w_dev) {
-    e = u_done ? launch_hv_rows(S, S.host_in.ptr, w_dev, fp64, 0, n, false, S.stream)
+    e = u_done ? launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, w_dev, fp64, 0, n, S.stream)
                : launch_hv(S, S.host_in.ptr, w_dev, fp64, S.stream);
   } else if (S.col && n >= (1 << 20)) {
     // rows in row order: the w rows of chunk c go back to the host while the
@@ -598,9 +598,11 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
     for (int c = 0; c < kChunks && e == cudaSuccess; ++c)
       if (!S.chunk_done[c]) e = cudaEventCreateWithFlags(&S.chunk_done[c], cudaEventDisableTiming);
     const size_t elem = fp64 ? 16 : 8;
+    if (e == cudaSuccess && !u_done) e = launch_u(S, S.host_in.ptr, S.ubuf.ptr, fp64, S.stream);
     for (int c = 0; c < kChunks && e == cudaSuccess; ++c) {
-      const int64_t r0 = n * c / kChunks, r1 = n * (c + 1) / kChunks;
-      e = launch_hv_rows(S, S.host_in.ptr, S.host_out.ptr, fp64, r0, r1, c == 0 && !u_done, S.stream);
+      // whole slices of 32 rows
+      const int64_t r0 = n * c / kChunks / 32 * 32, r1 = c + 1 == kChunks ? n : n * (c + 1) / kChunks / 32 * 32;
+      e = launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, S.host_out.ptr, fp64, r0, r1, S.stream);
       if (e == cudaSuccess) e = cudaEventRecord(S.chunk_done[c], S.stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(S.copy_stream, S.chunk_done[c], 0);
       if (e == cudaSuccess)
@@ -610,7 +612,7 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(S.copy_stream);
   } else {
     if (e == cudaSuccess)
-      e = u_done ? launch_hv_rows(S, S.host_in.ptr, S.host_out.ptr, fp64, 0, n, false, S.stream)
+      e = u_done ? launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, S.host_out.ptr, fp64, 0, n, S.stream)
                  : launch_hv(S, S.host_in.ptr, S.host_out.ptr, fp64, S.stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(w, S.host_out.ptr, bytes, cudaMemcpyDeviceToHost, S.stream);
   }

@@ -34,6 +34,7 @@
 
 #include "../../include/edgpu.h"
 #include "blas1.cuh"
+#include "csr_row.cuh"
 #include "edg_sector.cuh"
 #include "tridiag.cuh"
 
@@ -53,32 +54,34 @@ __device__ __forceinline__ double2 cconjmul(double2 a, double2 b) {  // conj(a) 
   return make_double2(a.x * b.x + a.y * b.y, a.x * b.y - a.y * b.x);
 }
 
-// H[j*n + i] += H_ij from the stored rows (one thread per row i)
+// H[j*n + i] += H_ij from the stored rows: a thread per row, a warp per slice
+// (csr_row.cuh)
 __global__ void k_dense_rows(const uint64_t* __restrict__ row_ptr, const uint32_t* __restrict__ col,
                              const uint16_t* __restrict__ vid, int cb, const double2* __restrict__ vtab,
                              const double* __restrict__ ezz, const uint8_t* __restrict__ lid,
                              const double* __restrict__ nrm, const double* __restrict__ nrm_inv, int64_t n,
                              double2* __restrict__ H) {
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const double ni = nrm[lid[i]];
-    for (uint64_t t = row_ptr[i]; t < row_ptr[i + 1]; ++t) {
-      const uint32_t e = col[t];
-      uint32_t j;
-      int id;
-      if (vid) {
-        j = e;
-        id = vid[t];
-      } else {
-        j = e & ((1u << cb) - 1u);
-        id = (int)(e >> cb);
+  const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t i = base + threadIdx.x;
+    const Slice s = slice_at(row_ptr, i, n);
+    const double ni = i < n ? nrm[lid[i]] : 0.0;
+    uint64_t at = s.base;
+    for (int k = 0; k < s.mx; ++k) {
+      const uint32_t m = __ballot_sync(0xffffffffu, s.len > k);
+      if (s.len > k) {
+        const uint64_t t = at + __popc(m & lt);
+        const uint32_t e = col[t];
+        const uint32_t j = vid ? e : e & ((1u << cb) - 1u);
+        const double2 c = vtab[vid ? (uint32_t)vid[t] : e >> cb];
+        const double sc = ni * nrm_inv[lid[j]];
+        double2* h = H + (int64_t)j * n + i;
+        h->x += c.x * sc;
+        h->y += c.y * sc;
       }
-      const double2 c = vtab[id];
-      const double s = ni * nrm_inv[lid[j]];
-      double2* h = H + (int64_t)j * n + i;
-      h->x += c.x * s;
-      h->y += c.y * s;
+      at += __popc(m);
     }
-    H[i * n + i].x += ezz[i];
+    if (i < n) H[i * n + i].x += ezz[i];
   }
 }
 

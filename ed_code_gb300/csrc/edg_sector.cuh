@@ -86,7 +86,7 @@ struct Sector {
   cudaEvent_t chunk_done[8] = {};
   // Lanczos work area (allocated on first use)
   DeviceBuffer lz_work;
-  // stored targets (targets.cu): CSR rows of (column, value id)
+  // stored targets (targets.cu): rows of (column, value id), by slices of 32 rows (csr_row.cuh)
   uint64_t* row_ptr = nullptr;  // n_p + 1
   uint32_t* col = nullptr;      // column, or column | value id << pack_cb
   uint16_t* vid = nullptr;      // value ids; null when the entries are packed
@@ -98,10 +98,10 @@ struct Sector {
   DeviceBuffer ubuf;            // u = v / norm scratch
   DeviceBuffer ublk;            // the same for edg_hv_block's interleaved vectors
   size_t targets_bytes = 0;
-  int csr_lpr = 16;             // lanes per CSR row (8, 16 or 32): edg_sector_tune
-  int csr_pol = 1;              // cache policy of the CSR loads (1 or 2): edg_sector_tune
-  int csr_cps = 0;              // CTAs per SM of the CSR kernel (0: as many as fit): edg_sector_tune
-  int csr_pipe = 0;             // 1: the CSR kernel loads the next rows' entries ahead: edg_sector_tune
+  int csr_lpr = 8;              // 8, 16 or 32: csr_lpr / 2 entries of a row in flight: edg_sector_tune
+  int csr_pol = 1;              // cache policy of the row loads (1 or 2): edg_sector_tune
+  int csr_cps = 0;              // CTAs per SM of the row kernel (0: as many as fit): edg_sector_tune
+  int csr_pipe = 1;             // 1: the row kernel loads the next entries ahead: edg_sector_tune
 };
 
 // basis.cu
@@ -153,8 +153,10 @@ void free_targets(Sector& S);
 cudaError_t launch_hv_stored(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st);
 // hv_block.cu: W = H V for nv = 2 or 4 vectors interleaved by row, u the n_p x nv scratch
 cudaError_t launch_hv_block(const Sector& S, const void* v, void* w, int nv, bool fp64, void* u, cudaStream_t st);
-// stored rows in row order: rows [r0, r1) of H*v, with the u = v/norm pass first when with_u
-cudaError_t launch_hv_rows(const Sector& S, const void* v, void* w, bool fp64, int64_t r0, int64_t r1, bool with_u,
+// stored rows: u = v / norm, and rows [r0, r1) of w = H v from v and u (r0 a
+// multiple of 32)
+cudaError_t launch_u(const Sector& S, const void* v, void* u, bool fp64, cudaStream_t st);
+cudaError_t launch_hv_rows(const Sector& S, const void* v, const void* u, void* w, bool fp64, int64_t r0, int64_t r1,
                            cudaStream_t st);
 // stored rows: u = v / norm and v_dst = v from a v_src the device reads in
 // place (mapped page-locked host memory)

@@ -12,8 +12,8 @@
 // id above the column when both fit (4 bytes), else a u32 column and a u16
 // id (6 bytes).  Rows also keep their diagonal Ezz.
 //
-// H*v is then a CSR SpMV with a value dictionary (one warp per row, lanes
-// over the row's entries):
+// H*v is then a sparse matrix-vector product with a value dictionary, a warp
+// per slice of 32 rows (csr_row.cuh, hv_rows.cuh):
 //     w_i = norm_i * sum_t vtab[vid_t] * u[col_t] + Ezz_i * v_i,
 //     u_j = v_j / norm_j (a streaming pass before the row loop).
 // This stores the Hamiltonian's structure (4 bytes per nonzero, 56 GB for the
@@ -35,14 +35,14 @@
 
 #include "csr_row.cuh"
 #include "hv_common.cuh"
+#include "hv_rows.cuh"
 
 namespace edg {
 
 namespace {
 
-constexpr int kWarpsPerBlock = 8;
-constexpr int kTgtThreads = 32 * kWarpsPerBlock;
 constexpr int kPassThreads = 128;
+constexpr int kMaxRowSlots = 256;  // a row has at most one entry per flip group
 constexpr int kMaxChPerGroup = 4;
 
 // A flip group as the passes below stage it: what a row needs to find out
@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const u
                                                            const uint64_t* __restrict__ row_ptr,
                                                            uint32_t* __restrict__ col, uint16_t* __restrict__ vid) {
   __shared__ SectorParams P;
+  __shared__ uint2 slots[kFill ? kPassThreads / 32 : 1][kFill ? kMaxRowSlots : 1];
   extern __shared__ __align__(16) uint8_t sm[];
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
     reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
@@ -195,7 +196,20 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const u
     bool uniq = false;
     uint32_t cnt = 0;
     double fac = 0.0;
-    if (kFill && live) pos = row_ptr[i];
+    uint2* slot = slots[kFill ? threadIdx.x >> 5 : 0];
+    if (kFill) {
+      // where the slice's slots start, and which rows have them (csr_row.cuh)
+      const Slice sl = slice_at(row_ptr, i, n_p);
+      uint32_t at = 0;
+      __syncwarp();
+      for (int k = 0; k < sl.mx; ++k) {
+        const uint32_t m = __ballot_sync(0xffffffffu, sl.len > k);
+        if ((threadIdx.x & 31) == 0) slot[k] = make_uint2(at, m);
+        at += __popc(m);
+      }
+      __syncwarp();
+      pos = sl.base;
+    }
     if (kOrb >= kOrbPacked) {
       // s is a representative: its top row is at its rotation minimum and no
       // row has a smaller one.  When it is the only row that reaches it and is
@@ -246,13 +260,14 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const u
           int variant = (int)((s >> gr.a) & 1u);
           for (int m = gr.ch_begin, b = 1; m < gr.ch_end; ++m, ++b) variant |= (int)((s >> H.z[m]) & 1u) << b;
           const uint32_t id = __ldg(remap + (gr.off + variant) * P.n_cls + P.g2cls[o.g]);
+          const uint2 sk = slot[cnt++];
+          const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
           if (cb) {
-            col[pos] = (uint32_t)j | (id << cb);
+            col[p] = (uint32_t)j | (id << cb);
           } else {
-            col[pos] = (uint32_t)j;
-            vid[pos] = (uint16_t)id;
+            col[p] = (uint32_t)j;
+            vid[p] = (uint16_t)id;
           }
-          ++pos;
         }
       }
     }
@@ -397,102 +412,6 @@ __global__ void k_u_scale_in(const typename CT2<Real>::T* __restrict__ v, const 
   }
 }
 
-// CSR SpMV with a value dictionary: 32/LPR rows per warp, a warp's row
-// groups a grid stride apart.  kFmt: kSplit or kPacked entries (csr_row.cuh),
-// cb the column bits of a packed entry.  kPipe sets how far a warp loads
-// ahead of the group it sums:
-//   0: the next group's offsets;
-//   1: also the next group's head entries, so their DRAM latency overlaps
-//      the current group's gathers instead of preceding them.
-// (Prefetching the next group's gather targets into L2 as well
-// (prefetch.global.L2) measured 121 ms against 60.6 ms at 36 sites: the
-// extra L2 requests cost more than the earlier start gains.)
-// The sums are the same bits either way.  (Loading the next group's gathers
-// as well, two groups' gathers in flight per warp, measured slower at 36
-// sites: 74.7 ms against 60.6 ms at 2 CTAs per SM.)
-template <typename Real, int LPR, bool kSmemTab, int kPol, int kFmt, int kPipe>
-__global__ void __launch_bounds__(kTgtThreads) k_hv_csr(const uint64_t* __restrict__ row_ptr,
-                                                        const uint32_t* __restrict__ col,
-                                                        const uint16_t* __restrict__ vid, int cb,
-                                                        const typename CT2<Real>::T* __restrict__ vtab, int n_vals,
-                                                        const double* __restrict__ ezz,
-                                                        const uint8_t* __restrict__ lid,
-                                                        const double* __restrict__ nrm_tab, int64_t row0,
-                                                        int64_t n_p, const typename CT2<Real>::T* __restrict__ v,
-                                                        const typename CT2<Real>::T* __restrict__ u,
-                                                        typename CT2<Real>::T* __restrict__ w) {
-  // rows [row0, n_p)
-  using CT = typename CT2<Real>::T;
-  constexpr int kRows = 32 / LPR;  // rows per warp
-  constexpr int kU = head_entries<LPR>();
-  extern __shared__ __align__(16) uint8_t sm[];
-  __shared__ Real nrm[65];
-  CT* tab = reinterpret_cast<CT*>(sm);
-  for (int k = threadIdx.x; k < 65; k += blockDim.x) nrm[k] = (Real)nrm_tab[k];
-  if (kSmemTab)
-    for (int k = threadIdx.x; k < n_vals; k += blockDim.x) tab[k] = vtab[k];
-  __syncthreads();
-  const CT* vt = kSmemTab ? tab : vtab;
-  const int lane = threadIdx.x & 31, sl = lane % LPR, sub = lane / LPR;
-  const int64_t warp = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int64_t n_warps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-  const int64_t stride = n_warps * kRows;
-  const unsigned long long* rp = reinterpret_cast<const unsigned long long*>(row_ptr);
-  const uint64_t pf = kPol == 2 ? l2_evict_first() : 0, pl = l2_evict_last();
-  auto offsets = [&](int64_t r, uint64_t& b, uint64_t& e) {
-    b = e = 0;
-    if (r < n_p) {
-      b = __ldg(rp + r);
-      e = __ldg(rp + r + 1);
-    }
-  };
-  auto store = [&](int64_t r, Real ar, Real ai) {
-    if (sl == 0 && r < n_p) {
-      w[r] = row_out(ar, ai, nrm[lid[r]], (Real)ezz[r], v[r]);
-    }
-  };
-  int64_t i = row0 + warp * kRows + sub;
-  uint64_t beg, end, beg1, end1;
-  offsets(i, beg, end);
-  offsets(i + stride, beg1, end1);
-  if (kPipe == 0) {
-    for (int64_t base = row0 + warp * kRows; base < n_p; base += stride) {
-      Real ar, ai;
-      csr_row<Real, LPR, kSmemTab, kPol, kFmt>(beg, end, sl, col, vid, cb, vt, u, ar, ai);
-      store(i, ar, ai);
-      i += stride;
-      beg = beg1;
-      end = end1;
-      offsets(i + stride, beg1, end1);
-    }
-  } else {
-    uint32_t e[kU];
-    uint16_t h[kU];
-    csr_head<LPR, kFmt, kPol>(beg, end, sl, col, vid, pf, e, h);
-    for (int64_t base = row0 + warp * kRows; base < n_p; base += stride) {
-      // group k+2's offsets, group k+1's head, then group k's gathers
-      uint64_t beg2, end2;
-      offsets(i + 2 * stride, beg2, end2);
-      uint32_t en[kU];
-      uint16_t hn[kU];
-      csr_head<LPR, kFmt, kPol>(beg1, end1, sl, col, vid, pf, en, hn);
-      Real ar, ai;
-      csr_finish<Real, LPR, kSmemTab, kPol, kFmt>(beg, end, sl, col, vid, cb, vt, u, pf, pl, e, h, ar, ai);
-      store(i, ar, ai);
-      i += stride;
-      beg = beg1;
-      end = end1;
-      beg1 = beg2;
-      end1 = end2;
-#pragma unroll
-      for (int q = 0; q < kU; ++q) {
-        e[q] = en[q];
-        h[q] = hn[q];
-      }
-    }
-  }
-}
-
 // Grid of a grid-stride kernel: the CTAs that fit on every SM at once, at most
 // cap per SM when cap > 0, no more than the work needs.
 template <typename K>
@@ -508,65 +427,36 @@ int grid_for(K kernel, size_t smem, int64_t work, int threads, int cap = 0) {
   return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
 }
 
-const double* params_field(const Sector& S, size_t offset) {
-  return reinterpret_cast<const double*>(reinterpret_cast<const char*>(S.dP) + offset);
-}
-
-// rows [r0, r1); u = v / norm first when with_u
-template <typename Real, int LPR, int kPol, int kFmt, int kPipe>
-cudaError_t launch_csr_lpr(const Sector& S, const void* v, void* w, cudaStream_t st, int64_t r0, int64_t r1,
-                           bool with_u) {
-  using CT = typename CT2<Real>::T;
-  const int64_t n = S.P.n_p;
-  if (with_u)
-    k_u_scale<Real><<<(int)std::min<int64_t>((n + 255) / 256, 152 * 32), 256, 0, st>>>(
-        reinterpret_cast<const CT*>(v), S.lid, params_field(S, offsetof(SectorParams, nrm_inv)), n,
-        reinterpret_cast<CT*>(S.ubuf.ptr));
-  const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
-  const size_t tab_bytes = sizeof(CT) * S.n_vals;
-  const double* nrm = params_field(S, offsetof(SectorParams, nrm));
-  if (r1 <= r0) return cudaGetLastError();
-  const int64_t threads_needed = ((r1 - r0) * LPR + 31) / 32 * 32;
-  if (tab_bytes <= 96 * 1024) {
-    auto kern = k_hv_csr<Real, LPR, true, kPol, kFmt, kPipe>;
-    kern<<<grid_for(kern, tab_bytes, threads_needed, kTgtThreads, S.csr_cps), kTgtThreads, tab_bytes, st>>>(
-        S.row_ptr, S.col, S.vid, S.pack_cb, tab, S.n_vals, S.ezz, S.lid, nrm, r0, r1, reinterpret_cast<const CT*>(v),
-        reinterpret_cast<const CT*>(S.ubuf.ptr), reinterpret_cast<CT*>(w));
-  } else {
-    auto kern = k_hv_csr<Real, LPR, false, kPol, kFmt, kPipe>;
-    kern<<<grid_for(kern, 0, threads_needed, kTgtThreads, S.csr_cps), kTgtThreads, 0, st>>>(
-        S.row_ptr, S.col, S.vid, S.pack_cb, tab, S.n_vals, S.ezz, S.lid, nrm, r0, r1, reinterpret_cast<const CT*>(v),
-        reinterpret_cast<const CT*>(S.ubuf.ptr), reinterpret_cast<CT*>(w));
-  }
-  return cudaGetLastError();
-}
-
+// The row kernel's tuned choices as template arguments: entries of a row in
+// flight (csr_lpr / 2: 4, 8 or 16; at most 8 in FP64, whose entries are twice
+// as large), cache policy, entry format, pipelining.  A value table too large
+// for shared memory is read through L1 with 8 entries in flight.
 template <typename Real, int kPol, int kFmt>
-cudaError_t launch_csr_f(const Sector& S, const void* v, void* w, cudaStream_t st, int64_t r0, int64_t r1,
-                         bool with_u) {
-  switch (S.csr_pipe * 3 + (S.csr_lpr == 8 ? 0 : S.csr_lpr == 16 ? 1 : 2)) {
-    case 0: return launch_csr_lpr<Real, 8, kPol, kFmt, 0>(S, v, w, st, r0, r1, with_u);
-    case 1: return launch_csr_lpr<Real, 16, kPol, kFmt, 0>(S, v, w, st, r0, r1, with_u);
-    case 2: return launch_csr_lpr<Real, 32, kPol, kFmt, 0>(S, v, w, st, r0, r1, with_u);
-    case 3: return launch_csr_lpr<Real, 8, kPol, kFmt, 1>(S, v, w, st, r0, r1, with_u);
-    case 4: return launch_csr_lpr<Real, 16, kPol, kFmt, 1>(S, v, w, st, r0, r1, with_u);
-    default: return launch_csr_lpr<Real, 32, kPol, kFmt, 1>(S, v, w, st, r0, r1, with_u);
+cudaError_t launch_rows_f(const Sector& S, const void* v, const void* u, void* w, int64_t r0, int64_t r1,
+                          cudaStream_t st) {
+  constexpr int kMost = sizeof(Real) == 4 ? 16 : 8;
+  if (sizeof(typename CT2<Real>::T) * S.n_vals > 96 * 1024)
+    return launch_rows_k<Real, 1, false, kPol, kFmt, 8, 8, false>(S, v, u, w, r0, r1, st);
+  if (S.csr_pipe) switch (S.csr_lpr) {
+      case 8: return launch_rows_k<Real, 1, true, kPol, kFmt, 4, 4, true>(S, v, u, w, r0, r1, st);
+      case 16: return launch_rows_k<Real, 1, true, kPol, kFmt, 8, 8, true>(S, v, u, w, r0, r1, st);
+      default: return launch_rows_k<Real, 1, true, kPol, kFmt, kMost, kMost, true>(S, v, u, w, r0, r1, st);
+    }
+  switch (S.csr_lpr) {
+    case 8: return launch_rows_k<Real, 1, true, kPol, kFmt, 4, 4, false>(S, v, u, w, r0, r1, st);
+    case 16: return launch_rows_k<Real, 1, true, kPol, kFmt, 8, 8, false>(S, v, u, w, r0, r1, st);
+    default: return launch_rows_k<Real, 1, true, kPol, kFmt, kMost, kMost, false>(S, v, u, w, r0, r1, st);
   }
-}
-
-template <typename Real, int kPol>
-cudaError_t launch_csr_p(const Sector& S, const void* v, void* w, cudaStream_t st, int64_t r0, int64_t r1,
-                         bool with_u) {
-  return S.pack_cb ? launch_csr_f<Real, kPol, kPacked>(S, v, w, st, r0, r1, with_u)
-                   : launch_csr_f<Real, kPol, kSplit>(S, v, w, st, r0, r1, with_u);
 }
 
 template <typename Real>
-cudaError_t launch_csr_t(const Sector& S, const void* v, void* w, cudaStream_t st, int64_t r0 = 0,
-                         int64_t r1 = -1, bool with_u = true) {
-  if (r1 < 0) r1 = S.P.n_p;
-  return S.csr_pol == 2 ? launch_csr_p<Real, 2>(S, v, w, st, r0, r1, with_u)
-                        : launch_csr_p<Real, 1>(S, v, w, st, r0, r1, with_u);
+cudaError_t launch_rows_t(const Sector& S, const void* v, const void* u, void* w, int64_t r0, int64_t r1,
+                          cudaStream_t st) {
+  if (S.pack_cb)
+    return S.csr_pol == 2 ? launch_rows_f<Real, 2, kPacked>(S, v, u, w, r0, r1, st)
+                          : launch_rows_f<Real, 1, kPacked>(S, v, u, w, r0, r1, st);
+  return S.csr_pol == 2 ? launch_rows_f<Real, 2, kSplit>(S, v, u, w, r0, r1, st)
+                        : launch_rows_f<Real, 1, kSplit>(S, v, u, w, r0, r1, st);
 }
 
 int64_t gcd64(int64_t a, int64_t b) {
@@ -607,7 +497,7 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     err = "stored targets do not cover ChCh terms";
     return EDG_ERR_UNSUPPORTED;
   }
-  if (P.n_groups > 256) {
+  if (P.n_groups > kMaxRowSlots) {
     err = "stored targets need at most 256 flip groups";
     return EDG_ERR_UNSUPPORTED;
   }
@@ -811,15 +701,16 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   return e == cudaSuccess ? EDG_OK : EDG_ERR_CUDA;
 }
 
-// Lanes per CSR row, cache policy, CTAs per SM and pipelining.  lpr in
-// {8, 16, 32} fixes the lanes; 0 times every lane count.  First every (lanes,
-// pipelining 0/1, CTA cap in {as many as fit, 4, 3, 2, 1}) with cache policy 2,
-// then the best of those with policy 1.  Each combination runs twice (FP32;
-// once on sectors whose launch takes over 5 ms) after one warm-up launch, and
-// the fastest is kept.  The CTA cap matters because the gathers reuse u
-// through L2: fewer rows in flight keep their targets' window of u smaller.
-// ms_out[k] receives the best time of lane count 8, 16, 32 (-1 when not
-// timed).
+// Entries in flight (lanes per row / 2), cache policy, CTAs per SM and
+// pipelining.  lpr in {8, 16, 32} fixes the first; 0 times all of them.  First
+// every (lanes, pipelining 0/1, CTA cap in {as many as fit, 4, 3, 2, 1}) with
+// cache policy 1, the faster one at 24 to 36 sites (392 us against 482 us at 30
+// sites, 54.8 ms against 61.8 ms at 36), then the best of those with policy 2.
+// Each combination runs twice (FP32; once on sectors whose launch takes over
+// 5 ms) after one warm-up launch, and the fastest is kept.  The CTA cap matters
+// because the gathers reuse u through L2: fewer rows in flight keep their
+// targets' window of u smaller.  ms_out[k] receives the best time of lane
+// count 8, 16, 32 (-1 when not timed).
 int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out) {
   if (!S.col) {
     if (chosen) *chosen = 0;
@@ -854,7 +745,7 @@ int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out) {
   };
   const int cand[3] = {8, 16, 32};
   const int caps[5] = {0, 4, 3, 2, 1};
-  int best = 16, best_cps = 0, best_pipe = 0;
+  int best = 8, best_cps = 0, best_pipe = 1;
   float best_ms = 1e30f;
   for (int k = 0; k < 3; ++k) {
     if (ms_out) ms_out[k] = -1;
@@ -862,7 +753,7 @@ int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out) {
     for (int pipe = 0; pipe < 2; ++pipe) {
       for (int c = 0; c < 5; ++c) {
         S.csr_lpr = cand[k];
-        S.csr_pol = 2;
+        S.csr_pol = 1;
         S.csr_cps = caps[c];
         S.csr_pipe = pipe;
         const float ms = time_it();
@@ -879,11 +770,11 @@ int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out) {
   S.csr_lpr = best;
   S.csr_cps = best_cps;
   S.csr_pipe = best_pipe;
-  S.csr_pol = 1;
-  const float ms1 = time_it();
+  S.csr_pol = 2;
+  const float ms2 = time_it();
   const int k = best == 8 ? 0 : best == 16 ? 1 : 2;
-  if (ms_out && ms1 < ms_out[k]) ms_out[k] = ms1;
-  if (ms1 >= best_ms) S.csr_pol = 2;
+  if (ms_out && ms2 < ms_out[k]) ms_out[k] = ms2;
+  if (ms2 >= best_ms) S.csr_pol = 1;
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   cudaFree(v);
@@ -892,9 +783,20 @@ int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out) {
   return cudaGetLastError() == cudaSuccess ? EDG_OK : EDG_ERR_CUDA;
 }
 
-cudaError_t launch_hv_rows(const Sector& S, const void* v, void* w, bool fp64, int64_t r0, int64_t r1, bool with_u,
+cudaError_t launch_u(const Sector& S, const void* v, void* u, bool fp64, cudaStream_t st) {
+  const int64_t n = S.P.n_p;
+  const int grid = (int)std::min<int64_t>((n + 255) / 256, 152 * 32);
+  const double* nrm_inv = params_field(S, offsetof(SectorParams, nrm_inv));
+  if (fp64)
+    k_u_scale<double><<<grid, 256, 0, st>>>(static_cast<const double2*>(v), S.lid, nrm_inv, n, static_cast<double2*>(u));
+  else
+    k_u_scale<float><<<grid, 256, 0, st>>>(static_cast<const float2*>(v), S.lid, nrm_inv, n, static_cast<float2*>(u));
+  return cudaGetLastError();
+}
+
+cudaError_t launch_hv_rows(const Sector& S, const void* v, const void* u, void* w, bool fp64, int64_t r0, int64_t r1,
                            cudaStream_t st) {
-  return fp64 ? launch_csr_t<double>(S, v, w, st, r0, r1, with_u) : launch_csr_t<float>(S, v, w, st, r0, r1, with_u);
+  return fp64 ? launch_rows_t<double>(S, v, u, w, r0, r1, st) : launch_rows_t<float>(S, v, u, w, r0, r1, st);
 }
 
 cudaError_t launch_u_in(const Sector& S, const void* v_src, void* v_dst, bool fp64, cudaStream_t st) {
@@ -911,7 +813,8 @@ cudaError_t launch_u_in(const Sector& S, const void* v_src, void* v_dst, bool fp
 }
 
 cudaError_t launch_hv_stored(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st) {
-  return fp64 ? launch_csr_t<double>(S, v, w, st) : launch_csr_t<float>(S, v, w, st);
+  const cudaError_t e = launch_u(S, v, S.ubuf.ptr, fp64, st);
+  return e == cudaSuccess ? launch_hv_rows(S, v, S.ubuf.ptr, w, fp64, 0, S.P.n_p, st) : e;
 }
 
 }  // namespace edg

@@ -70,8 +70,9 @@ class GpuSector:
         return True
 
     def tune(self, lanes_per_row: int = 0):
-        """Choose the lanes per stored row and the cache policy of its loads by
-        timing them on this sector (0: all lane counts; 8/16/32: that count).
+        """Choose the stored-row kernel's entries in flight (lanes_per_row / 2),
+        cache policy, CTAs per SM and pipelining by timing them on this sector
+        (0: all; 8/16/32: that lanes_per_row).
         Returns (lanes, [best ms for 8, 16, 32], -1 where not timed); the
         choices are also in ``info["lanes_per_row"]``, ``info["cache_policy"]``,
         ``info["ctas_per_sm"]`` and ``info["pipelined"]``."""
@@ -82,7 +83,8 @@ class GpuSector:
         return ch.value, ms
 
     def set_rows(self, lanes_per_row: int, cache_policy: int, ctas_per_sm: int = 0, pipelined: int = 0) -> None:
-        """Fix the stored-row kernel's lanes per row (8/16/32), cache policy (1/2),
+        """Fix the stored-row kernel's entries in flight (lanes_per_row / 2 with
+        lanes_per_row 8, 16 or 32), cache policy (1/2),
         CTAs per SM (0: as many as fit) and pipelining (0/1)."""
         N.check(N.lib().edg_sector_set_rows(self._h, int(lanes_per_row), int(cache_policy), int(ctas_per_sm),
                                             int(pipelined)))

@@ -68,14 +68,14 @@ typedef struct {
   int64_t n_configs;     /* C(N, n_ones) */
   int64_t device_bytes;  /* device memory held by the sector */
   int64_t n_targets;     /* stored nonzeros (0: H*v searches on the fly) */
-  int lanes_per_row;     /* stored-row H*v: lanes of a warp per row (edg_sector_tune) */
+  int lanes_per_row;     /* stored-row H*v: lanes_per_row / 2 entries of a row in flight (edg_sector_tune) */
   int cache_policy;      /* stored-row H*v: 1 streaming row loads, 2 L2 evict-first row loads */
   int L3, kz;            /* third translation's cycle length and momentum (1, 0 in 2-D) */
   int entry_bytes;       /* bytes of one stored nonzero: 4 (column and value id packed in one
                             u32), 6 (u32 column + u16 value id), 0 without stored rows */
   int n_values;          /* distinct values of the stored rows' value table */
   int ctas_per_sm;       /* stored-row H*v: CTAs per SM (0: as many as fit) */
-  int pipelined;         /* stored-row H*v: 1 when the next rows' entries load during the gathers */
+  int pipelined;         /* stored-row H*v: 1 when the next entries load during the gathers */
 } edg_sector_info;
 
 const char* edg_last_error(void);
@@ -134,12 +134,14 @@ int edg_hv(edg_sector* s, const void* v, void* w, int dtype, void* stream);
 int edg_sector_build_targets(edg_sector* s, int64_t max_bytes);
 int edg_sector_free_targets(edg_sector* s);
 
-/* Lanes of a warp per stored row (8, 16 or 32, i.e. 4, 2 or 1 rows per warp),
- * the cache policy of the row loads, the CTAs per SM (as many as fit, or at
- * most 4, 3, 2 or 1: fewer rows in flight keep the gathered part of v in L2)
- * and pipelining (1: the next rows' entries loaded while the current rows
- * gather), timed on this sector: a nonzero lanes_per_row fixes the lanes and times the rest, 0 times
- * every lane count.  The fastest is kept.  *chosen receives the lanes, ms
+/* Entries of a row in flight (lanes_per_row / 2: 4, 8 or 16; the rows are
+ * stored by slices of 32 and a lane sums a row, so the parameter keeps only its
+ * name from the layout with several lanes per row), the cache policy of the row
+ * loads, the CTAs per SM (as many as fit, or at most 4, 3, 2 or 1: fewer rows
+ * in flight keep the gathered part of v in L2) and pipelining (1: a row's next
+ * entries loaded while the current ones gather), timed on this sector: a
+ * nonzero lanes_per_row fixes the first and times the rest, 0 times all.  The
+ * fastest is kept.  *chosen receives the lanes, ms
  * (NULL allowed) the best time of 8, 16 and 32 lanes in that order (-1: not
  * timed); edg_sector_info reports the four choices. */
 int edg_sector_tune(edg_sector* s, int lanes_per_row, int* chosen, double* ms);
@@ -270,7 +272,7 @@ int edg_solve_mixed(edg_sector* s, const edg_mixed_opts* opts, double* eigs, dou
  * has been polled.  One thread drives a batch. */
 typedef struct {
   int tile_rows;      /* rows per CTA tile (0: 1024) */
-  int lanes_per_row;  /* lanes per stored row: 8, 16 or 32 (0: 8) */
+  int lanes_per_row;  /* 8, 16 or 32 (0: 8): lanes_per_row / 2 entries of a stored row in flight */
   int check_every;    /* steps between convergence tests (0: 10) */
   int reorth;         /* 0: reorthogonalise every step; 1: partial reorthogonalisation
                          (only the steps where estimates of the lost orthogonality,
@@ -313,12 +315,12 @@ int edg_batch_add(edg_batch* b, edg_sector* s, const edg_batch_request* req);
 int edg_batch_step(edg_batch* b, int n_steps);
 /* Autotuner of the batch kernels: times `steps` steps of the segments added so
  * far (before the batch's first step) for tiles of 256, 1024, 4096 and 16384
- * rows with 8 and 16 lanes per stored row, keeps the fastest for the rest of
+ * rows with lanes_per_row 8 and 16, keeps the fastest for the rest of
  * the batch and returns it (NULL allowed); ms (NULL allowed) receives the 8
  * trial times per step, tiles major.  The segments are then put back at their
  * seeded start, so the results are those of an untuned batch created with the
- * chosen options.  A segment's arithmetic depends on the tile size and the
- * lanes per row (the order of its sums), not on the other segments. */
+ * chosen options.  A segment's arithmetic depends on the tile size (the
+ * order of its sums over the rows), not on the other segments. */
 int edg_batch_tune(edg_batch* b, int steps, int* tile_rows, int* lanes_per_row, double* ms);
 /* Withdraw the live segment with this tag: its memory is released now and its
  * result (status EDG_ERR_CANCELLED, no levels) comes back through

@@ -35,3 +35,36 @@ def test_stored_rows_of_every_search_match_oracle(cuda_device, Lx, Ly, Sz, k, J2
     assert sec.build_targets()
     assert sec.info["n_targets"] == sec.count_offdiag()
     assert np.abs(sec.sHv(v) - w).max() / max(1.0, np.abs(w).max()) <= 1e-13
+
+
+@pytest.mark.parametrize("Lx,Ly,Sz,k", [
+    (4, 3, 0, (1, 2)),   # 75 rows: a last slice of 11 rows, 8 warps a slice
+    (5, 4, 0, (0, 0)),   # 290 slices: 4 warps
+    (6, 4, 4, (2, 1)),   # 956 slices: 2 warps
+    (6, 4, 2, (3, 0)),   # 2,556 slices: 1 warp
+])
+def test_row_sums_of_every_split_match_oracle(cuda_device, Lx, Ly, Sz, k):
+    """A slice's slots are split among 8, 4, 2 or 1 warps by the sector's size:
+    each against the oracle (FP64, and FP32 at the other tests' 2e-5), and the
+    block kernel's bits against the single vector's."""
+    import torch
+
+    from ed_code_gb300 import lattice as L
+    from ed_code_gb300 import sector
+
+    model = L.make_model(L.TorusSpec("triangular", Lx, Ly, Jz=0.7, Ch=0.3), Sz, *k, bowties=False)
+    ref = O.OracleSector(model)
+    sec = sector.GpuSector(model)
+    assert sec.build_targets()
+    v = O.splitmix_vector(sec.n_p, 6)
+    w = ref.hv(v)
+    scale = max(1.0, np.abs(w).max())
+    for dt, tol in ((np.complex128, 1e-13), (np.complex64, 2e-5)):
+        one = sec.sHv(v.astype(dt), dtype=dt)
+        assert np.abs(one - w).max() / scale <= tol
+        V = torch.from_numpy(np.stack([v.astype(dt)] * 4, axis=1).copy()).cuda()
+        W = torch.empty_like(V)
+        sec.hv_block(V, W)
+        torch.cuda.synchronize()
+        for q in range(4):
+            assert np.array_equal(W.cpu().numpy()[:, q], one), (dt, q)
