@@ -32,6 +32,7 @@
 #include "blas1.cuh"
 #include "edg_sector.cuh"
 #include "lanczos_common.cuh"
+#include "multidot.cuh"
 #include "tridiag.cuh"
 
 namespace edg {
@@ -44,82 +45,90 @@ namespace {
 using cplx = std::complex<double>;
 
 // ---------------------------------------------------------------- kernels ---
-template <typename T>
-__global__ void __launch_bounds__(kRedThreads) k_dotc_partial(const T* __restrict__ V, int64_t ld,
-                                                              const T* __restrict__ x, int64_t n,
-                                                              double* __restrict__ part) {
-  // part[(k*kRedBlocks + b)*2 + {0,1}] = partial sum of conj(V_k) x, k = blockIdx.y
-  const T* a = V + (int64_t)blockIdx.y * ld;
-  Acc sr, si;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const cd p = VecTraits<T>::load(a, i), q = VecTraits<T>::load(x, i);
-    sr.add(p.re * q.re + p.im * q.im);
-    si.add(p.re * q.im - p.im * q.re);
-  }
-  __shared__ double rr[kRedThreads], ri[kRedThreads];
-  rr[threadIdx.x] = sr.value();
-  ri[threadIdx.x] = si.value();
+// The last CTA's sums of a streaming kernel's compensated per-thread sums, in
+// CTA order (multidot.cuh's tickets): true there, sum[] in all its threads.
+// part: kN gridDim.x doubles.
+template <int kN>
+__device__ __forceinline__ bool close_acc(const Acc (&r)[kN], double* part, int* cnt, double (&sum)[kN]) {
+  __shared__ double sm[kN][kRedThreads], tot[kN];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto over_threads = [&](int k) {  // by one warp
+    double x = 0;
+#pragma unroll
+    for (int q = 0; q < kRedThreads / 32; ++q) x += sm[k][32 * q + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    return x;
+  };
+#pragma unroll
+  for (int k = 0; k < kN; ++k) sm[k][threadIdx.x] = r[k].value();
   __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      rr[threadIdx.x] += rr[threadIdx.x + h];
-      ri[threadIdx.x] += ri[threadIdx.x + h];
-    }
-    __syncthreads();
+  if (wid < kN) {
+    const double x = over_threads(wid);
+    if (lane == 0) part[(int64_t)wid * gridDim.x + blockIdx.x] = x;
   }
-  if (threadIdx.x == 0) {
-    const int64_t o = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 2;
-    part[o] = rr[0];
-    part[o + 1] = ri[0];
+  if (!md_last(cnt, gridDim.x)) return false;
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    double x = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) x += __ldcg(part + (int64_t)k * gridDim.x + i);
+    sm[k][threadIdx.x] = x;
   }
+  __syncthreads();
+  if (wid < kN) {
+    const double x = over_threads(wid);
+    if (lane == 0) tot[wid] = x;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kN; ++k) sum[k] = tot[k];
+  return true;
 }
 
-// One CTA per vector: sum its kRedBlocks partials in a fixed order.  mode 0:
-// the complex sum to out[2k], out[2k+1]; mode 1: out[0] = sqrt(Re sum) (a
-// norm); mode 2: out[0] = 1 / sqrt(Re sum) (the normalising factor).
-__global__ void __launch_bounds__(kRedThreads) k_dot_finish(const double* __restrict__ part, int nb,
-                                                            double* __restrict__ out, int mode) {
-  const double* p = part + (int64_t)blockIdx.x * nb * 2;
-  __shared__ double rr[kRedThreads], ri[kRedThreads];
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    a += p[2 * i];
-    b += p[2 * i + 1];
-  }
-  rr[threadIdx.x] = a;
-  ri[threadIdx.x] = b;
-  __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      rr[threadIdx.x] += rr[threadIdx.x + h];
-      ri[threadIdx.x] += ri[threadIdx.x + h];
+// w -= beta v' (v' and beta the previous step's, or nullptr), then <v|w> into
+// alpha (complex): lanczos.cpp:237-238 in one pass.
+__global__ void __launch_bounds__(kRedThreads) k_beta_alpha(double2* __restrict__ w, const double2* __restrict__ vprev,
+                                                            const double* __restrict__ beta,
+                                                            const double2* __restrict__ v, int64_t n,
+                                                            double* __restrict__ part, int* __restrict__ cnt,
+                                                            double* __restrict__ alpha) {
+  const double b = vprev ? *beta : 0.0;
+  Acc s[2];
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    double2 y = w[i];
+    const double2 x = v[i];
+    if (vprev) {
+      const double2 p = vprev[i];
+      y.x -= b * p.x;
+      y.y -= b * p.y;
+      w[i] = y;
     }
-    __syncthreads();
+    s[0].add(x.x * y.x + x.y * y.y);
+    s[1].add(x.x * y.y - x.y * y.x);
   }
-  if (threadIdx.x == 0) {
-    if (mode == 0) {
-      out[2 * blockIdx.x] = rr[0];
-      out[2 * blockIdx.x + 1] = ri[0];
-    } else if (mode == 1) {
-      out[0] = sqrt(rr[0]);
-    } else {
-      out[0] = 1.0 / sqrt(rr[0]);
-    }
-  }
+  double sum[2];
+  if (close_acc<2>(s, part, cnt, sum) && threadIdx.x < 2) alpha[threadIdx.x] = sum[threadIdx.x];
 }
 
-// y -= c x with a device scalar c: complex (c[0], c[1]) when cplx, else real c[0]
-template <typename T>
-__global__ void k_sub_scaled(T* __restrict__ y, const T* __restrict__ x, const double* __restrict__ c, bool cplx,
-                             int64_t n) {
-  const double cr = c[0], ci = cplx ? c[1] : 0.0;
+// w -= alpha v (alpha complex), vs = v, and |w| into *nrm.
+__global__ void __launch_bounds__(kRedThreads) k_alpha_norm(double2* __restrict__ w, const double2* __restrict__ v,
+                                                            const double* __restrict__ alpha,
+                                                            double2* __restrict__ vs, int64_t n,
+                                                            double* __restrict__ part, int* __restrict__ cnt,
+                                                            double* __restrict__ nrm) {
+  const double ar = alpha[0], ai = alpha[1];
+  Acc s[1];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const cd xv = VecTraits<T>::load(x, i);
-    cd yv = VecTraits<T>::load(y, i);
-    yv.re -= cr * xv.re - ci * xv.im;
-    yv.im -= cr * xv.im + ci * xv.re;
-    VecTraits<T>::store(y, i, yv);
+    double2 y = w[i];
+    const double2 x = v[i];
+    y.x -= ar * x.x - ai * x.y;
+    y.y -= ar * x.y + ai * x.x;
+    w[i] = y;
+    vs[i] = x;
+    s[0].add(y.x * y.x + y.y * y.y);
   }
+  double sum[1];
+  if (close_acc<1>(s, part, cnt, sum) && threadIdx.x == 0) *nrm = sqrt(sum[0]);
 }
 
 // y = s x with a real device scalar: s = c[0] (inv false) or 1 / c[0] (inv true)
@@ -172,6 +181,9 @@ __global__ void k_combine(T* __restrict__ out, const T* __restrict__ V, int64_t 
   }
 }
 
+// CTAs of the streaming kernels that end in a sum: four an SM
+constexpr int kRedCtas = 152 * 4;
+int grid_red(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kRedCtas)); }
 int grid_of(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16)); }
 
 // ------------------------------------------------------------ vector ops ---
@@ -180,38 +192,33 @@ int grid_of(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n +
 // the next kernel: a Lanczos step queues its kernels without waiting.
 struct Blas {
   cudaStream_t st;
-  double* part = nullptr;  // partials for up to kMaxDots vectors
+  double* part = nullptr;  // partials for up to k_max vectors
+  int* cnt = nullptr;      // ticket counters, zero between launches
   double* res = nullptr;   // finished dots of up to 2 kMaxDots vectors (device)
   double* scal = nullptr;  // small device scalars
   static constexpr int kMaxDots = 1024;
-  cudaError_t init(cudaStream_t s) {
+  cudaError_t init(cudaStream_t s, int k_max) {
     st = s;
-    cudaError_t e = cudaMalloc(&part, sizeof(double) * 2 * kRedBlocks * kMaxDots);
+    cudaError_t e = cudaMalloc(&part, sizeof(double) * std::max<size_t>(md_part(k_max), 2 * kRedCtas));
+    if (e == cudaSuccess) e = cudaMalloc(&cnt, sizeof(int) * md_cnt(k_max));
+    if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, sizeof(int) * md_cnt(k_max), s);
     if (e == cudaSuccess) e = cudaMalloc(&res, sizeof(double) * 4 * kMaxDots);
     if (e == cudaSuccess) e = cudaMalloc(&scal, sizeof(double) * 8);
     return e;
   }
   ~Blas() {
     cudaFree(part);
+    cudaFree(cnt);
     cudaFree(res);
     cudaFree(scal);
   }
   // out[k] = <V_k | x> = sum conj(V_k) x for k < K (complex, device), all
   // computed before anything changes x
-  template <typename T>
-  void dots(const T* V, int64_t ld, int K, const T* x, int64_t n, double* out) {
-    for (int k0 = 0; k0 < K; k0 += kMaxDots) {
-      const int kk = std::min(kMaxDots, K - k0);
-      k_dotc_partial<T><<<dim3(kRedBlocks, kk), kRedThreads, 0, st>>>(V + (int64_t)k0 * ld, ld, x, n, part);
-      k_dot_finish<<<kk, kRedThreads, 0, st>>>(part, kRedBlocks, out + 2 * k0, 0);
-    }
+  void dots(const double2* V, int64_t ld, int K, const double2* x, int64_t n, double* out) {
+    mdot<Md64>(st, V, ld, K, x, n, part, cnt, out, kMdComplex);
   }
-  // out[0] = sqrt(<x|x>) (mode 1) or 1 / sqrt(<x|x>) (mode 2)
-  template <typename T>
-  void norm(const T* x, int64_t n, double* out, int mode) {
-    k_dotc_partial<T><<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(x, 0, x, n, part);
-    k_dot_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, out, mode);
-  }
+  // out[0] = 1 / sqrt(<x|x>)
+  void inv_norm(const double2* x, int64_t n, double* out) { mdot<Md64>(st, x, 0, 1, x, n, part, cnt, out, kMdInvNorm); }
   // y -= sum_k q_k V_k, q complex on the device
   template <typename T>
   void sub_multi(T* y, const T* V, int64_t ld, const double* q, int K, int64_t n) {
@@ -233,7 +240,7 @@ void orth(Blas& B, double2* v, const double2* V, int64_t ld, int K, int64_t n) {
 
 // normalize (lanczos.cpp:50-55)
 void normalize(Blas& B, double2* v, int64_t n) {
-  B.norm(v, n, B.scal, 2);
+  B.inv_norm(v, n, B.scal);
   k_scale_dev<double2><<<grid_of(n), 256, 0, B.st>>>(v, v, B.scal, false, n);
 }
 
@@ -248,6 +255,36 @@ void log_line(const edg_solver_opts& o, const char* fmt, ...) {
   o.log_fn(o.log_ctx, buf);
 }
 
+// Device times of a cycle's steps without waiting in between: events before and
+// after each H v and before its reorthogonalisation, read at the cycle's end.
+struct StepClock {
+  std::vector<cudaEvent_t> ev;
+  size_t used = 0;
+  void mark(cudaStream_t st) {
+    if (used == ev.size()) {
+      cudaEvent_t e = nullptr;
+      if (cudaEventCreate(&e) != cudaSuccess) return;
+      ev.push_back(e);
+    }
+    cudaEventRecord(ev[used++], st);
+  }
+  // the stream has been waited for: three marks a step and one at the end
+  void sum(double& hv, double& ortho) {
+    for (size_t k = 0; k + 3 < used; k += 3) {
+      float a = 0, b = 0;
+      if (cudaEventElapsedTime(&a, ev[k], ev[k + 1]) == cudaSuccess &&
+          cudaEventElapsedTime(&b, ev[k + 2], ev[k + 3]) == cudaSuccess) {
+        hv += 1e-3 * a;
+        ortho += 1e-3 * b;
+      }
+    }
+    used = 0;
+  }
+  ~StepClock() {
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  }
+};
+
 int solve_lanczos(Sector& S, const edg_solver_opts& o, double* eigs, int64_t cap, int64_t* n_out, double* evecs,
                   int64_t evecs_cap, edg_solver_stats* stats) {
   const int64_t n = S.P.n_p;
@@ -261,7 +298,7 @@ int solve_lanczos(Sector& S, const edg_solver_opts& o, double* eigs, int64_t cap
   int iterations = o.iterations;
   cudaStream_t st = S.stream;
   Blas B;
-  cudaError_t ce = B.init(st);
+  cudaError_t ce = B.init(st, (int)std::max<int64_t>(std::min<int64_t>(iterations, n), how_many));
   if (ce != cudaSuccess) return fail(EDG_ERR_NOMEM, "Lanczos: scratch allocation");
   // device storage: v_p, w, the Krylov vectors of a cycle, earlier
   // eigenvectors, and T: alpha (complex), beta (beta[0] = 0, beta[j] the
@@ -305,6 +342,7 @@ int solve_lanczos(Sector& S, const edg_solver_opts& o, double* eigs, int64_t cap
   const auto t_start = clk::now();
   double t_hv = 0, t_ortho = 0;
   int64_t hv_calls = 0;
+  StepClock clock;
   std::vector<double> all_eigs;
   double eig0 = 0;
   cudaMemsetAsync(beta, 0, sizeof(double) * (max_it + 2), st);
@@ -317,29 +355,33 @@ int solve_lanczos(Sector& S, const edg_solver_opts& o, double* eigs, int64_t cap
       normalize(B, vp, n);
       int n_vs = 0;
       bool stop_cycle = false;
+      const bool middle = cycle != 0 && cycle != o.ncycles - 1;
+      bool known = false;  // eig0 is this cycle's lowest value after its last step
       for (int it = 0; it < iterations && !stop_cycle; ++it) {
-        auto t0 = clk::now();
+        clock.mark(st);
         if ((ce = launch_hv(S, vp, w, true, st)) != cudaSuccess) break;
-        if ((ce = cudaStreamSynchronize(st)) != cudaSuccess) break;
-        t_hv += std::chrono::duration<double>(clk::now() - t0).count();
+        clock.mark(st);
         ++hv_calls;
         // w -= beta_it v_{it-1}; alpha = conj(zdotc(w, v_p)) = <v_p|w> (lanczos.cpp:237-238)
-        if (it != 0) k_sub_scaled<double2><<<grid_of(n), 256, 0, st>>>(w, vs + (int64_t)(it - 1) * n, beta + it,
-                                                                       false, n);
-        B.dots(vp, 0, 1, w, n, alpha + 2 * it);
-        k_sub_scaled<double2><<<grid_of(n), 256, 0, st>>>(w, vp, alpha + 2 * it, true, n);
-        cudaMemcpyAsync(vs + (int64_t)n_vs * n, vp, sizeof(double2) * n, cudaMemcpyDeviceToDevice, st);
+        k_beta_alpha<<<grid_red(n), kRedThreads, 0, st>>>(w, it != 0 ? vs + (int64_t)(it - 1) * n : nullptr, beta + it,
+                                                          vp, n, B.part, B.cnt, alpha + 2 * it);
+        // w -= alpha v_p, v_p stored, beta = |w|
+        k_alpha_norm<<<grid_red(n), kRedThreads, 0, st>>>(w, vp, alpha + 2 * it, vs + (int64_t)n_vs * n, n, B.part,
+                                                          B.cnt, beta + it + 1);
         ++n_vs;
-        B.norm(w, n, beta + it + 1, 1);  // beta = |w|
         k_scale_dev<double2><<<grid_of(n), 256, 0, st>>>(vp, w, beta + it + 1, true, n);  // v_p = w / beta
-        auto t1 = clk::now();
+        clock.mark(st);
         orth(B, vp, prev, n, num, n);
         if (cycle == o.ncycles - 1) orth(B, vp, vs, n, n_vs, n);
         normalize(B, vp, n);
-        // lowest eigenvalue of T (diagonal Re(alpha), off-diagonal beta), on the device
+        // Lowest eigenvalue of T (diagonal Re(alpha), off-diagonal beta), on the
+        // device: wanted after every step by the middle cycles' convergence test
+        // and by the log, else only after a cycle's last step (below, with its
+        // eigenvector), and then the steps are queued without a wait.
+        known = o.log_fn || middle;
+        if (!known) continue;
         if ((ce = lowest(it + 1, false, eig0)) != cudaSuccess) break;
-        t_ortho += std::chrono::duration<double>(clk::now() - t1).count();
-        if (cycle != 0 && cycle != o.ncycles - 1 && it > 1) {
+        if (middle && it > 1) {
           log_line(o, "Eigs[0]      = %+.15f", eig0);
           log_line(o, "Previous Eig = %+.15f", previous_eig);
           if (std::fabs(eig0 - previous_eig) < o.tol) {
@@ -360,7 +402,13 @@ int solve_lanczos(Sector& S, const edg_solver_opts& o, double* eigs, int64_t cap
       // Ritz vector from the stored Krylov vectors (lanczos.cpp:311-320): the
       // eigenvector of T on the device, then v_p = sum_k y_k vs_k
       double th = 0;
+      clock.mark(st);
       if ((ce = lowest(n_vs, true, th)) != cudaSuccess) break;
+      if (!known) {
+        eig0 = th;
+        if (cycle != o.ncycles - 1) previous_eig = eig0;
+      }
+      clock.sum(t_hv, t_ortho);
       k_combine<double2><<<grid_of(n), 256, sizeof(double) * n_vs, st>>>(vp, vs, n, y, n_vs, n);
       orth(B, vp, prev, n, num, n);
       normalize(B, vp, n);

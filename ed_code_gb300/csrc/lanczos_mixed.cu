@@ -43,6 +43,7 @@
 #include "blas1.cuh"
 #include "edg_sector.cuh"
 #include "ff.cuh"
+#include "multidot.cuh"
 #include "tridiag.cuh"
 #include "lanczos_common.cuh"
 
@@ -81,6 +82,7 @@ struct P32 {
   using Real = float;
   using A = FFAcc;
   using S = FFScalar;
+  using M = Md32;
   static constexpr bool kFp64 = false;
   static __device__ __forceinline__ float axpy2(float x, S a, float u, S b, float w) { return ff_axpy2(x, a, u, b, w); }
   static __device__ __forceinline__ float scale(float x, S s) { return fmaf(x, s.l, __fmul_rn(x, s.h)); }
@@ -90,6 +92,7 @@ struct P64 {
   using Real = double;
   using A = DAcc;
   using S = DScalar;
+  using M = Md64;
   static constexpr bool kFp64 = true;
   static __device__ __forceinline__ double axpy2(double x, S a, double u, S b, double w) {
     return fma(-b.v, w, fma(-a.v, u, x));
@@ -104,148 +107,93 @@ __device__ __forceinline__ typename P::V mk(typename P::Real x, typename P::Real
   return r;
 }
 
-// partial sums of sum conj(a) b: exact (P32) or FP64 (P64) products summed per
-// thread, FP64 across threads; part[(k*gridDim.x + b)*2 + {0,1}], k =
-// blockIdx.y selects a = V + k*ld
-template <class P>
-__global__ void __launch_bounds__(kRedThreads) k_dot(const typename P::V* __restrict__ V, int64_t ld,
-                                                     const typename P::V* __restrict__ x, int64_t n,
-                                                     double* __restrict__ part, const double* run = nullptr,
-                                                     const int* kf = nullptr, int k0 = 0) {
-  if (run && *run == 0.0) return;
-  if (kf && k0 + (int)blockIdx.y < *kf) return;  // before this step's Gram-Schmidt range
-  const typename P::V* a = V + (int64_t)blockIdx.y * ld;
-  typename P::A sr, si;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const typename P::V p = a[i], q = x[i];
-    sr.add_prod(p.x, q.x);
-    sr.add_prod(p.y, q.y);
-    si.add_prod(p.x, q.y);
-    si.sub_prod(p.y, q.x);
-  }
-  __shared__ double rr[kRedThreads], ri[kRedThreads];
-  rr[threadIdx.x] = sr.value();
-  ri[threadIdx.x] = si.value();
+// The sums of kN accumulators over the grid: per CTA (one warp per accumulator,
+// which costs 13 FP64 additions a CTA instead of 40: FP64 issue is 16 clocks),
+// then, in the CTA that finishes last, over all CTAs in CTA order.  True there,
+// where all threads have the sums.  part: kN gridDim.x doubles.
+template <int kN, class A>
+__device__ __forceinline__ bool close_sums(const A (&r)[kN], double* part, int* cnt, double (&sum)[kN]) {
+  __shared__ double sm[kN][kRedThreads];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  auto over_threads = [&](int k) {  // by one warp
+    double x = 0;
+#pragma unroll
+    for (int q = 0; q < kRedThreads / 32; ++q) x += sm[k][32 * q + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    return x;
+  };
+#pragma unroll
+  for (int k = 0; k < kN; ++k) sm[k][threadIdx.x] = r[k].value();
   __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      rr[threadIdx.x] += rr[threadIdx.x + h];
-      ri[threadIdx.x] += ri[threadIdx.x + h];
-    }
-    __syncthreads();
+  if (wid < kN) {
+    const double x = over_threads(wid);
+    if (lane == 0) part[(int64_t)wid * gridDim.x + blockIdx.x] = x;
   }
-  if (threadIdx.x == 0) {
-    const int64_t o = ((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 2;
-    part[o] = rr[0];
-    part[o + 1] = ri[0];
+  if (!md_last(cnt, gridDim.x)) return false;
+#pragma unroll
+  for (int k = 0; k < kN; ++k) {
+    double x = 0;
+    for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) x += __ldcg(part + (int64_t)k * gridDim.x + i);
+    sm[k][threadIdx.x] = x;
   }
-}
-
-// Sum the partials of vector k (one CTA per k); mode 0: complex result to
-// out[2k], mode 1: real part to out[0], mode 2: sqrt of the real part to out[0].
-__global__ void __launch_bounds__(kRedThreads) k_finish(const double* __restrict__ part, int nb, double* out,
-                                                        int mode, const double* run = nullptr,
-                                                        const int* kf = nullptr, int k0 = 0) {
-  if (run && *run == 0.0) return;
-  if (kf && k0 + (int)blockIdx.x < *kf) return;
-  const double* p = part + (int64_t)blockIdx.x * nb * 2;
-  __shared__ double rr[kRedThreads], ri[kRedThreads];
-  double a = 0, b = 0;
-  for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-    a += p[2 * i];
-    b += p[2 * i + 1];
-  }
-  rr[threadIdx.x] = a;
-  ri[threadIdx.x] = b;
   __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      rr[threadIdx.x] += rr[threadIdx.x + h];
-      ri[threadIdx.x] += ri[threadIdx.x + h];
-    }
-    __syncthreads();
+  __shared__ double tot[kN];
+  if (wid < kN) {
+    const double x = over_threads(wid);
+    if (lane == 0) tot[wid] = x;
   }
-  if (threadIdx.x == 0) {
-    if (mode == 0) {
-      out[2 * blockIdx.x] = rr[0];
-      out[2 * blockIdx.x + 1] = ri[0];
-    } else if (mode == 1) {
-      out[0] = rr[0];
-    } else {
-      out[0] = sqrt(rr[0]);
-    }
-  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < kN; ++k) sum[k] = tot[k];
+  return true;
 }
 
 // w = w - alpha v - beta vprev (FP64 alpha/beta; P32: float-float, one final
-// rounding to the FP32 storage), and partial sums of |w|^2 of the stored values.
+// rounding to the FP32 storage), and |w|^2 of the stored values into *w2 or its
+// root into *nrm; with omega, the CTA that closes it goes on to the estimates of partial
+// reorthogonalisation (pro_step; state = {force, kf, full steps}).
 template <class P>
 __global__ void __launch_bounds__(kRedThreads) k_step(typename P::V* __restrict__ w, const typename P::V* __restrict__ v,
                                                       const typename P::V* __restrict__ vprev,
                                                       const double* __restrict__ alpha,
                                                       const double* __restrict__ beta, int64_t n,
-                                                      double* __restrict__ part) {
+                                                      double* __restrict__ part, int* __restrict__ cnt, double* w2,
+                                                      double* nrm, int j, double* omega, int ld, int* state) {
   using V = typename P::V;
-  const typename P::S a(*alpha), b(vprev ? *beta : 0.0);
-  typename P::A s;
+  const typename P::S a(alpha[j]), b(vprev ? beta[j] : 0.0);
+  typename P::A s[1];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const V wi = w[i], vi = v[i];
     const V pi = vprev ? vprev[i] : mk<P>(0, 0);
     const V o = mk<P>(P::axpy2(wi.x, a, vi.x, b, pi.x), P::axpy2(wi.y, a, vi.y, b, pi.y));
     w[i] = o;
-    s.add_prod(o.x, o.x);
-    s.add_prod(o.y, o.y);
+    s[0].add_prod(o.x, o.x);
+    s[0].add_prod(o.y, o.y);
   }
-  __shared__ double rr[kRedThreads];
-  rr[threadIdx.x] = s.value();
-  __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) rr[threadIdx.x] += rr[threadIdx.x + h];
-    __syncthreads();
-  }
+  double x[1];
+  if (!close_sums<1>(s, part, cnt, x)) return;
   if (threadIdx.x == 0) {
-    part[2 * blockIdx.x] = rr[0];
-    part[2 * blockIdx.x + 1] = 0.0;
+    if (nrm) *nrm = sqrt(x[0]);
+    else *w2 = x[0];
   }
-}
-
-// Block sums of kQ complex accumulators into part[(k*gridDim.x + b)*2 + {0,1}].
-template <int kQ, class A>
-__device__ __forceinline__ void block_partials(const A (&r)[kQ], const A (&i)[kQ], double* part) {
-  __shared__ double rr[kRedThreads], ri[kRedThreads];
-  for (int k = 0; k < kQ; ++k) {
-    rr[threadIdx.x] = r[k].value();
-    ri[threadIdx.x] = i[k].value();
-    __syncthreads();
-    for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-      if ((int)threadIdx.x < h) {
-        rr[threadIdx.x] += rr[threadIdx.x + h];
-        ri[threadIdx.x] += ri[threadIdx.x + h];
-      }
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) {
-      const int64_t o = ((int64_t)k * gridDim.x + blockIdx.x) * 2;
-      part[o] = rr[0];
-      part[o + 1] = ri[0];
-    }
-    __syncthreads();
-  }
+  if (omega) pro_step(alpha, beta, j, x[0], omega, ld, state, state + 1, state + 2);
 }
 
 // The local form's step in one pass: w = w - alpha v - beta vprev as k_step,
-// then the partials of <v|w> and <vprev|w> (0 without vprev) for the local
-// reorthogonalisation, k = 0 and 1 in k_finish's layout.
+// then <v|w> and <vprev|w> (0 without vprev) for the local reorthogonalisation
+// into q[0..3].
 template <class P>
 __global__ void __launch_bounds__(kRedThreads) k_step_dots(typename P::V* __restrict__ w,
                                                            const typename P::V* __restrict__ v,
                                                            const typename P::V* __restrict__ vprev,
                                                            const double* __restrict__ alpha,
                                                            const double* __restrict__ beta, int64_t n,
-                                                           double* __restrict__ part) {
+                                                           double* __restrict__ part, int* __restrict__ cnt,
+                                                           double* __restrict__ q) {
   using V = typename P::V;
   const typename P::S a(*alpha), b(vprev ? *beta : 0.0);
-  typename P::A r[2], im[2];
+  typename P::A r[4];  // <v|w>, <vprev|w>: real and imaginary parts
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const V wi = w[i], vi = v[i];
     const V pi = vprev ? vprev[i] : mk<P>(0, 0);
@@ -253,28 +201,30 @@ __global__ void __launch_bounds__(kRedThreads) k_step_dots(typename P::V* __rest
     w[i] = o;
     r[0].add_prod(vi.x, o.x);
     r[0].add_prod(vi.y, o.y);
-    im[0].add_prod(vi.x, o.y);
-    im[0].sub_prod(vi.y, o.x);
-    r[1].add_prod(pi.x, o.x);
-    r[1].add_prod(pi.y, o.y);
-    im[1].add_prod(pi.x, o.y);
-    im[1].sub_prod(pi.y, o.x);
+    r[1].add_prod(vi.x, o.y);
+    r[1].sub_prod(vi.y, o.x);
+    r[2].add_prod(pi.x, o.x);
+    r[2].add_prod(pi.y, o.y);
+    r[3].add_prod(pi.x, o.y);
+    r[3].sub_prod(pi.y, o.x);
   }
-  block_partials<2>(r, im, part);
+  double x[4];
+  if (close_sums<4>(r, part, cnt, x) && threadIdx.x < 4) q[threadIdx.x] = x[threadIdx.x];
 }
 
 // w -= q0 v + q1 vprev (q complex, device; arithmetic in the vectors'
-// precision, as k_sub) and the partials of |w|^2 in k_finish's layout.
+// precision, as k_sub), and |w| into *nrm when nrm is given.
 template <class P>
 __global__ void __launch_bounds__(kRedThreads) k_sub2_norm(typename P::V* __restrict__ w,
                                                            const typename P::V* __restrict__ v,
                                                            const typename P::V* __restrict__ vprev,
                                                            const double* __restrict__ q, int64_t n,
-                                                           double* __restrict__ part) {
+                                                           double* __restrict__ part, int* __restrict__ cnt,
+                                                           double* nrm) {
   using V = typename P::V;
   using R = typename P::Real;
   const R q0r = (R)q[0], q0i = (R)q[1], q1r = (R)q[2], q1i = (R)q[3];
-  typename P::A r[1], im[1];
+  typename P::A r[1];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const V y0 = w[i], vi = v[i];
     R re = fmr(-q0r, vi.x, fmr(q0i, vi.y, y0.x));
@@ -288,7 +238,9 @@ __global__ void __launch_bounds__(kRedThreads) k_sub2_norm(typename P::V* __rest
     r[0].add_prod(re, re);
     r[0].add_prod(ii, ii);
   }
-  block_partials<1>(r, im, part);
+  if (!nrm) return;
+  double x[1];
+  if (close_sums<1>(r, part, cnt, x) && threadIdx.x == 0) *nrm = sqrt(x[0]);
 }
 
 // dst = src / beta (dst may be src); P32: 1/beta as an FP32 head and tail
@@ -302,13 +254,14 @@ __global__ void k_scale_inv(typename P::V* dst, const typename P::V* src, const 
 }
 
 // y -= sum_k q_k V_k with q (complex, device) read into shared memory in the
-// vectors' precision.  The q_k are tiny against |y| once the vectors are
-// nearly orthogonal, so P32's FP32 arithmetic adds errors far below the FP32
-// rounding of y itself.
+// vectors' precision, and |y| into *nrm when nrm is given.  The q_k are tiny
+// against |y| once the vectors are nearly orthogonal, so P32's FP32 arithmetic
+// adds errors far below the FP32 rounding of y itself.
 template <class P>
-__global__ void k_sub(typename P::V* __restrict__ y, const typename P::V* __restrict__ V, int64_t ld,
-                      const double* __restrict__ q, int K, int64_t n, const double* run = nullptr,
-                      const int* kf = nullptr, int k0 = 0) {
+__global__ void __launch_bounds__(kRedThreads) k_sub(typename P::V* __restrict__ y, const typename P::V* __restrict__ V,
+                                                     int64_t ld, const double* __restrict__ q, int K, int64_t n,
+                                                     const double* run, const int* kf, int k0,
+                                                     double* __restrict__ part, int* __restrict__ cnt, double* nrm) {
   if (run && *run == 0.0) return;
   const int kb = kf ? max(0, *kf - k0) : 0;  // this step's range starts at V_kf
   using R = typename P::Real;
@@ -316,6 +269,7 @@ __global__ void k_sub(typename P::V* __restrict__ y, const typename P::V* __rest
   R* sq = reinterpret_cast<R*>(sraw);
   for (int k = threadIdx.x; k < 2 * K; k += blockDim.x) sq[k] = (R)q[k];
   __syncthreads();
+  typename P::A s[1];
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const typename P::V y0 = y[i];
     R re = y0.x, im = y0.y;
@@ -326,36 +280,12 @@ __global__ void k_sub(typename P::V* __restrict__ y, const typename P::V* __rest
       im = fmr(-qr, vv.y, fmr(-qi, vv.x, im));
     }
     y[i] = mk<P>(re, im);
+    s[0].add_prod(re, re);
+    s[0].add_prod(im, im);
   }
-}
-
-// Whether a classical Gram-Schmidt pass needs a second one (Daniel, Gragg,
-// Kaufman and Stewart's criterion): the first removed sum_k |q_k|^2 of
-// x's |x|^2; more than 1e-4 of it means x had a component along the V_k large
-// enough that the pass's own rounding matters, and the pass is repeated.
-// *run = 1.0 or 0.0 for the second pass's kernels.
-__global__ void __launch_bounds__(kRedThreads) k_cgs_decide(const double* __restrict__ q, int K,
-                                                            const double* __restrict__ xn2, double* run,
-                                                            const int* kf) {
-  __shared__ double sm[kRedThreads];
-  double a = 0;
-  for (int k = (kf ? *kf : 0) + threadIdx.x; k < K; k += blockDim.x)
-    a += q[2 * k] * q[2 * k] + q[2 * k + 1] * q[2 * k + 1];
-  sm[threadIdx.x] = a;
-  __syncthreads();
-  for (int h = kRedThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) sm[threadIdx.x] += sm[threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) *run = sm[0] > 1e-4 * *xn2 ? 1.0 : 0.0;
-}
-
-// Partial reorthogonalisation's estimates for this step (pro_step); state =
-// {force, kf, full steps}.
-__global__ void __launch_bounds__(kProThreads) k_pro(const double* __restrict__ alpha, const double* __restrict__ beta,
-                                                     int j, const double* __restrict__ w2, double* omega, int ld,
-                                                     int* state) {
-  pro_step(alpha, beta, j, *w2, omega, ld, state, state + 1, state + 2);
+  if (!nrm) return;
+  double a[1];
+  if (close_sums<1>(s, part, cnt, a) && threadIdx.x == 0) *nrm = sqrt(a[0]);
 }
 
 // Second pass of the resident-vector mode: X_e += sum_t y[e*m + j0 + t] V_{j0+t}
@@ -542,6 +472,10 @@ __global__ void __launch_bounds__(kRedThreads) k_rq_sum(const double* __restrict
   }
 }
 
+// CTAs of the streaming kernels that end in close_sums: eight an SM, as many as
+// are resident, so that the sums over a CTA's threads are paid once a slot
+constexpr int kRedCtas = 152 * 8;
+int grid_red(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, kRedCtas)); }
 int grid_n(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 16)); }
 
 struct Dev {
@@ -728,11 +662,14 @@ static int solve_mixed_t(Sector& S, const edg_mixed_opts& o, double* eigs, doubl
     cudaGetLastError();
   }
   if ((e = D.alloc(&w, (size_t)n)) != cudaSuccess) return fail(EDG_ERR_NOMEM, "mixed Lanczos: w");
-  const int64_t kparts = (int64_t)std::max(m + 1, 4) * kRedBlocks * 2;
+  // partials and ticket counters of the reductions (zero between launches)
+  const size_t kparts = std::max<size_t>(md_part(m + 1), 4 * kRedCtas);
+  int* cnt = nullptr;
   if ((e = D.alloc(&alpha, m + 1)) != cudaSuccess || (e = D.alloc(&beta, m + 2)) != cudaSuccess ||
       (e = D.alloc(&part, kparts)) != cudaSuccess || (e = D.alloc(&scal, 2 * (m + 2) + 2)) != cudaSuccess ||
-      (e = D.alloc(&lq, 4)) != cudaSuccess)
+      (e = D.alloc(&lq, 4)) != cudaSuccess || (e = D.alloc(&cnt, md_cnt(m + 1))) != cudaSuccess)
     return fail(EDG_ERR_NOMEM, "mixed Lanczos: scratch");
+  cudaMemsetAsync(cnt, 0, sizeof(int) * md_cnt(m + 1), st);
   cudaMemsetAsync(beta, 0, sizeof(double) * (m + 2), st);
   double* omega = nullptr;
   int* pstate = nullptr;  // {force, kf, full steps}
@@ -744,8 +681,7 @@ static int solve_mixed_t(Sector& S, const edg_mixed_opts& o, double* eigs, doubl
 
   auto vec = [&](int j) -> Vt* { return j < kept ? V + (int64_t)j * n : buf[(j - kept) % ring]; };
   auto norm_into = [&](const Vt* x, double* dst) {  // dst = |x| in FP64
-    k_dot<P><<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(x, 0, x, n, part);
-    k_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, dst, 2);
+    mdot<typename P::M>(st, x, 0, 1, x, n, part, cnt, dst, kMdNorm);
   };
   double t_hv = 0;
   int64_t hv_calls = 0;
@@ -778,10 +714,7 @@ static int solve_mixed_t(Sector& S, const edg_mixed_opts& o, double* eigs, doubl
       auto t0 = clk::now();
       if ((ce = launch_hv(S, vec(j), w, P::kFp64, st)) != cudaSuccess) return ce;
       ++hv_calls;
-      if (!second) {
-        k_dot<P><<<dim3(kRedBlocks, 1), kRedThreads, 0, st>>>(vec(j), 0, w, n, part);
-        k_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, alpha + j, 1);
-      }
+      if (!second) mdot<typename P::M>(st, vec(j), 0, 1, w, n, part, cnt, alpha + j, kMdReal);
       if (!reorth) {
         // Local reorthogonalisation of w against v_j and v_{j-1}, the vectors
         // still resident: it slows the growth of the copies that FP32 vectors
@@ -790,14 +723,16 @@ static int solve_mixed_t(Sector& S, const edg_mixed_opts& o, double* eigs, doubl
         // The second pass repeats it (the kernels are deterministic, so with
         // the same coefficients).
         const Vt* vp = j > 0 ? vec(j - 1) : nullptr;
-        k_step_dots<P><<<kRedBlocks, kRedThreads, 0, st>>>(w, vec(j), vp, alpha + j, beta + j, n, part);
-        k_finish<<<2, kRedThreads, 0, st>>>(part, kRedBlocks, lq, 0);
-        k_sub2_norm<P><<<kRedBlocks, kRedThreads, 0, st>>>(w, vec(j), vp, lq, n, part);
-        if (!second) k_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, beta + j + 1, 2);
+        k_step_dots<P><<<grid_red(n), kRedThreads, 0, st>>>(w, vec(j), vp, alpha + j, beta + j, n, part, cnt, lq);
+        k_sub2_norm<P><<<grid_red(n), kRedThreads, 0, st>>>(w, vec(j), vp, lq, n, part, cnt,
+                                                          second ? nullptr : beta + j + 1);
       } else {
-        k_step<P><<<kRedBlocks, kRedThreads, 0, st>>>(w, vec(j), j > 0 ? vec(j - 1) : nullptr, alpha + j, beta + j,
-                                                      n, part);
-        if (!second && (partial || (j + 1) % o.reorth_every == 0)) {
+        // |w|^2 into lq[0]; without reorthogonalisation this step its root is beta
+        const bool orth_now = !second && (partial || (j + 1) % o.reorth_every == 0);
+        k_step<P><<<grid_red(n), kRedThreads, 0, st>>>(w, vec(j), j > 0 ? vec(j - 1) : nullptr, alpha, beta, n, part, cnt,
+                                                     lq, orth_now ? nullptr : beta + j + 1, j, partial ? omega : nullptr, m + 2,
+                                                       pstate);
+        if (orth_now) {
           // Periodic reorthogonalisation in its two-vector form: between two
           // reorthogonalisations v_j has drifted too, so it is cleaned against
           // v_0..v_{j-1} first, then w against v_0..v_j.  (Cleaning w alone
@@ -809,31 +744,25 @@ static int solve_mixed_t(Sector& S, const edg_mixed_opts& o, double* eigs, doubl
           // it only now and then.  With partial reorthogonalisation the range
           // is v_kf..v_j, kf set on the device each step (pro_step): j - 1
           // (local) or 0 (full, when the estimates call for it).
-          auto cgs2 = [&](Vt* x, int K, const double* xn2, const int* kf) {
+          // |x| after the last pass that ran goes to nrm.
+          auto cgs2 = [&](Vt* x, int K, const double* xn2, const int* kf, double* nrm) {
             for (int pass = 0; pass < 2; ++pass) {
               const double* run = pass == 1 && xn2 ? lq + 1 : nullptr;
+              mdot<typename P::M>(st, V, n, K, x, n, part, cnt, scal, kMdComplex, run, kf,
+                                  pass == 0 && xn2 ? lq + 1 : nullptr, xn2);
               for (int k0 = 0; k0 < K; k0 += 512) {
                 const int kk = std::min(512, K - k0);
-                k_dot<P><<<dim3(kRedBlocks, kk), kRedThreads, 0, st>>>(V + (int64_t)k0 * n, n, x, n, part, run,
-                                                                       kf, k0);
-                k_finish<<<kk, kRedThreads, 0, st>>>(part, kRedBlocks, scal + 2 * k0, 0, run, kf, k0);
-                k_sub<P><<<grid_n(n), 256, sizeof(typename P::Real) * 2 * kk, st>>>(x, V + (int64_t)k0 * n, n,
-                                                                                    scal + 2 * k0, kk, n, run, kf, k0);
+                k_sub<P><<<grid_red(n), kRedThreads, sizeof(typename P::Real) * 2 * kk, st>>>(
+                    x, V + (int64_t)k0 * n, n, scal + 2 * k0, kk, n, run, kf, k0, part, cnt,
+                    k0 + kk == K ? nrm : nullptr);
               }
-              if (pass == 0 && xn2) k_cgs_decide<<<1, kRedThreads, 0, st>>>(scal, K, xn2, lq + 1, kf);
             }
           };
           if (!partial && o.reorth_every > 1 && j > 0) {
-            cgs2(vec(j), j, nullptr, nullptr);
-            norm_into(vec(j), scal + 2 * (m + 1));
+            cgs2(vec(j), j, nullptr, nullptr, scal + 2 * (m + 1));
             k_scale_inv<P><<<grid_n(n), 256, 0, st>>>(vec(j), vec(j), scal + 2 * (m + 1), n);
           }
-          k_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, lq, 1);  // |w|^2 after the step (k_step)
-          if (partial) k_pro<<<1, kProThreads, 0, st>>>(alpha, beta, j, lq, omega, m + 2, pstate);
-          cgs2(w, j + 1, lq, partial ? pstate + 1 : nullptr);
-          norm_into(w, beta + j + 1);
-        } else if (!second) {
-          k_finish<<<1, kRedThreads, 0, st>>>(part, kRedBlocks, beta + j + 1, 2);
+          cgs2(w, j + 1, lq, partial ? pstate + 1 : nullptr, beta + j + 1);
         }
       }
       if (j + 1 < m || second) k_scale_inv<P><<<grid_n(n), 256, 0, st>>>(vec(j + 1), w, beta + j + 1, n);
