@@ -37,7 +37,7 @@ constexpr double kPi = 3.14159265358979323846;
 static void free_sector(Sector& S) {
   free_targets(S);
   void* ptrs[] = {S.dP,   S.reps,    S.lid,         S.recs,         S.vrecs,       S.Ia,    S.Ib,
-                  S.groups, S.ch,   S.bows,    S.nk,          S.rots,         S.perms,       S.binom, S.host_in.ptr,
+                  S.groups, S.ch,   S.bows,    S.nk,          S.rots,         S.perms,       S.binom, S.host_in.ptr, S.values,
                   S.host_out.ptr, S.lz_work.ptr, S.ublk.ptr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -351,6 +351,35 @@ static int create_sector(const edg_model* m, int n_ones, int kx, int ky, int kz,
   e = cudaMalloc(&S.recs, sizeof(RankRec) * std::max<int64_t>(1, P.n_recs));
   if (e != cudaSuccess) return fail(EDG_ERR_NOMEM, "rank records: out of device memory");
   bytes += sizeof(RankRec) * std::max<int64_t>(1, P.n_recs);
+  // the value tables in one allocation: both tables first, they are the widest
+  ValueTables T;
+  if (value_tables(P, groups, ch, T) == EDG_OK) {
+    if (T.v64.empty()) {  // no flip at all: one value that no row has
+      T.v64.push_back(make_double2(0.0, 0.0));
+      T.v32.push_back(make_float2(0.f, 0.f));
+    }
+    std::vector<uint8_t> all;
+    auto put = [&](const void* src, size_t n) {
+      const size_t at = all.size();
+      all.resize(at + (n + 15) / 16 * 16);
+      std::memcpy(all.data() + at, src, n);
+      return at;
+    };
+    const size_t o64 = put(T.v64.data(), 16 * T.v64.size()), o32 = put(T.v32.data(), 8 * T.v32.size());
+    const size_t ov = put(T.voff.data(), 2 * T.voff.size()), oo = put(T.order.data(), 2 * T.order.size());
+    const size_t orm = put(T.remap.data(), 2 * T.remap.size());
+    uint8_t* dev = nullptr;
+    if ((e = upload(&dev, all.data(), all.size(), bytes)) != cudaSuccess) return cuda_fail(e, "value tables");
+    S.values = dev;
+    S.vtab64 = reinterpret_cast<double2*>(dev + o64);
+    S.vtab32 = reinterpret_cast<float2*>(dev + o32);
+    S.V.voff = reinterpret_cast<const uint16_t*>(dev + ov);
+    S.V.order = reinterpret_cast<const uint16_t*>(dev + oo);
+    S.V.remap = reinterpret_cast<const uint16_t*>(dev + orm);
+    S.n_vals = (int)T.v64.size();
+  } else {
+    S.values_err = T.why;
+  }
   if ((e = upload(&S.dP, &P, 1, bytes)) != cudaSuccess) return cuda_fail(e, "params");
   S.device_bytes = bytes;
 
@@ -455,7 +484,7 @@ int edg_sector_get_info(const edg_sector* s, edg_sector_info* info) {
   info->ctas_per_sm = s->s.col ? s->s.csr_cps : 0;
   info->pipelined = s->s.col ? s->s.csr_pipe : 0;
   info->entry_bytes = s->s.col ? (s->s.pack_cb ? 4 : 6) : 0;
-  info->n_values = s->s.n_vals;
+  info->n_values = s->s.col ? s->s.n_vals : 0;
   return EDG_OK;
 }
 

@@ -28,6 +28,9 @@ struct SectorView {
   const uint16_t* rots;    // torus: rotations reaching it
   const uint64_t* perms;   // walk: n_perm x n_chunks x 256 permutation chunk tables (T1, T2[, T3])
   const uint64_t* binom;   // (kMaxSites+1)^2 binomials
+  const uint16_t* voff;    // value tables: first variant of each group,
+  const uint16_t* order;   // the groups, high sites first,
+  const uint16_t* remap;   // and the value id of (variant, phase class)
   int n_chunks;
   int n_perm;              // 2, or 3 on a 3-D torus
   int row_bits;            // torus: Lx (table size 2^Lx)
@@ -73,6 +76,11 @@ struct Sector {
   uint16_t* rots = nullptr;
   uint64_t* perms = nullptr;
   uint64_t* binom = nullptr;
+  void* values = nullptr;       // value tables (value_tables), one allocation
+  double2* vtab64 = nullptr;    // in it: the distinct pair coefficient x phase values
+  float2* vtab32 = nullptr;
+  int n_vals = 0;               // 0: the tables do not cover the Hamiltonian (values_err)
+  std::string values_err;
   size_t device_bytes = 0;
   // host copies used by the adapters
   std::vector<int> T1, T2, T3;  // T3 empty in 2-D
@@ -92,9 +100,6 @@ struct Sector {
   uint16_t* vid = nullptr;      // value ids; null when the entries are packed
   int pack_cb = 0;              // column bits of a packed entry (0: split arrays)
   double* ezz = nullptr;        // diagonal of each row
-  double2* vtab64 = nullptr;    // value table: pair coefficient x phase class
-  float2* vtab32 = nullptr;
-  int n_vals = 0;
   DeviceBuffer ubuf;            // u = v / norm scratch
   DeviceBuffer ublk;            // the same for edg_hv_block's interleaved vectors
   size_t targets_bytes = 0;
@@ -147,6 +152,14 @@ struct MixedFinish {
 };
 void pick_levels(const std::vector<double>& rr, const std::vector<double>& th, const std::vector<int>& acc_h, int na,
                  int want, double* eigs, double* ritz, double* resid, std::vector<int>& keep);
+// targets.cu: see there
+struct ValueTables {
+  std::vector<uint16_t> voff, order, remap;
+  std::vector<double2> v64;
+  std::vector<float2> v32;
+  std::string why;
+};
+int value_tables(SectorParams& P, const std::vector<TermGroup>& groups, const std::vector<ChTerm>& ch, ValueTables& T);
 cudaError_t count_offdiag(const Sector& S, unsigned long long* nnz_dev, cudaStream_t st);
 int build_targets(Sector& S, int64_t max_bytes, std::string& err);
 void free_targets(Sector& S);

@@ -1,6 +1,12 @@
 // Matrix-free H*v in the momentum basis: the role of sHv (H_v.cpp:192-357).
 //
-// One thread owns one basis row i (coalesced loads of reps/lid/v and a
+// k_hv_free takes every Hamiltonian whose values fit the value tables
+// (targets.cu): a thread per row walks the flip groups as the stored rows'
+// build does (row_walk.cuh), leaves what it finds in shared memory and sums it
+// as the stored rows are summed (csr_row.cuh).  k_hv takes the rest: ChCh terms
+// and couplings of many values.
+//
+// k_hv: one thread owns one basis row i (coalesced loads of reps/lid/v and a
 // coalesced store of w).  Per row:
 //   * the anti-aligned flip groups are found 64 at a time as a bit mask
 //     (groups merge every bond and chirality term that flips the same pair);
@@ -20,7 +26,9 @@
 
 #include <algorithm>
 
+#include "csr_row.cuh"
 #include "hv_common.cuh"
+#include "row_walk.cuh"
 
 namespace edg {
 
@@ -137,6 +145,139 @@ __global__ void __launch_bounds__(kHvThreads, 4) k_hv(SectorView V, const typena
   }
 }
 
+// The matrix-free H*v over the value tables.  The warps of a CTA each take 32
+// neighbouring rows; the lanes go through the flip groups together, and a
+// target found goes into the lane's next slot of the warp's queue in shared
+// memory (column and value id).  When a lane's queue is full, or the groups are
+// through, the warp sums the slots as it would stored ones.  So the search runs
+// on rows that take the same turns, the gathers of several targets are in
+// flight together, and a target costs four FP64 multiply-adds (two when real)
+// instead of 16 FP64 instructions for its coefficient, phase, norm and product,
+// which was what bound it (FP64 pipe 83 % busy): 2,484 us -> 1,097 us at 28 sites in
+// FP64.  The gathered entries would need v / norm; with trivial stabilisers the
+// norms are one factor of the row, and the few targets with others are added
+// apart.
+constexpr int kFreeThreads = 128, kQueue = 16;
+
+// (r, i) += c x sc; a call, so that its FP64 instructions are not predicated
+// into every turn of the walk
+template <typename Real, typename CT>
+__device__ __noinline__ void add_rest(CT c, CT x, Real sc, Real& r, Real& i) {
+  r += (c.x * x.x - c.y * x.y) * sc;
+  i += (c.x * x.y + c.y * x.x) * sc;
+}
+
+template <typename Real>
+size_t free_smem_bytes(const Sector& S, int orb) {
+  return align16(pass_smem_bytes(S.P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm)) +
+         sizeof(typename CT2<Real>::T) * S.n_vals;
+}
+
+template <typename Real, int kOrb>
+__global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const typename CT2<Real>::T* __restrict__ vtab,
+                                                          int n_vals, int table_at,
+                                                          const typename CT2<Real>::T* __restrict__ v,
+                                                          typename CT2<Real>::T* __restrict__ w) {
+  using CT = typename CT2<Real>::T;
+  __shared__ SectorParams P;
+  __shared__ Real nrm[65], nrm_inv[65];
+  __shared__ uint32_t q_col[kFreeThreads / 32][kQueue][32];
+  __shared__ uint16_t q_id[kFreeThreads / 32][kQueue][32];
+  extern __shared__ __align__(16) uint8_t sm[];
+  for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
+    reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
+  __syncthreads();
+  const PassSmem H = stage_pass<kOrb>(V, P, sm);
+  CT* tab = reinterpret_cast<CT*>(sm + table_at);
+  for (int k = threadIdx.x; k < n_vals; k += blockDim.x) tab[k] = vtab[k];
+  for (int k = threadIdx.x; k < 65; k += blockDim.x) {
+    nrm[k] = (Real)P.nrm[k];
+    nrm_inv[k] = (Real)P.nrm_inv[k];
+  }
+  __syncthreads();
+  using St = typename OrbRows<kOrb>::T::State;
+  const int ng = P.n_groups, lane = threadIdx.x & 31;
+  auto& qc = q_col[threadIdx.x >> 5];
+  auto& qi = q_id[threadIdx.x >> 5];
+  const uint64_t pl = l2_evict_last();
+  const RowsView<Real> R{nullptr, nullptr, nullptr, tab, v, 0};
+  const int64_t n_p = P.n_p, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_p; base += stride) {
+    const int64_t i = base + threadIdx.x;
+    const bool live = i < n_p;
+    const St s = live ? (St)V.reps[i] : 0;  // no pair is anti-aligned past the end
+    CT vi;
+    vi.x = vi.y = 0;
+    int li = 1;
+    if (live) {
+      vi = v[i];
+      li = V.lid[i];
+    }
+    Real acc[partial_sums<Real>()][2];
+#pragma unroll
+    for (int a = 0; a < partial_sums<Real>(); ++a) acc[a][0] = acc[a][1] = 0;
+    Real rest_r = 0, rest_i = 0;  // targets with a stabiliser, by norm_1 / norm_j
+    uint64_t facs = 0;
+    int cnt = 0;
+    RowStart<kOrb> row;
+    row.set(s, P, H);
+    auto flush = [&]() {
+      const int mx = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);
+      __syncwarp();
+      for (int k = 0; k < mx; k += 4) {
+        uint32_t e[4], act = 0;
+        uint16_t h[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const bool has = k + q < cnt;
+          e[q] = has ? qc[k + q][lane] : 0u;
+          h[q] = has ? qi[k + q][lane] : (uint16_t)0;
+          act |= has ? 1u << q : 0u;
+        }
+        take_slots<Real, 1, kSplit, 4, 4>(R, e, h, act, 0xFFFFFFFFu, false, pl, acc);
+      }
+      __syncwarp();
+      cnt = 0;
+    };
+    for (int g = 0; g < ng; ++g) {
+      const PassGroup& gr = H.groups[g];
+      const St pm = (St)gr.mask, both = s & pm;
+      const bool anti = both != 0 && both != pm;
+      if (!__any_sync(0xffffffffu, anti)) continue;
+      if (anti) {
+        facs += gr.facadd;
+        bool known;
+        const Orbit o = target_orbit<kOrb, false>((St)(s ^ pm), gr, row, P, H, V.n_chunks, known);
+        const int64_t j = position(o, V, P);
+        if (j >= 0) {
+          const uint32_t id = value_id(s, gr, o.g, V, P, H);
+          if (o.stab == 1) {
+            qc[cnt][lane] = (uint32_t)j;
+            qi[cnt][lane] = (uint16_t)id;
+            ++cnt;
+          } else {
+            add_rest(tab[id], v[j], nrm_inv[o.stab] * nrm[1], rest_r, rest_i);
+          }
+        }
+      }
+      if (__any_sync(0xffffffffu, cnt == kQueue)) flush();
+    }
+    flush();
+    Real sum[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      constexpr int kAcc = partial_sums<Real>();
+#pragma unroll
+      for (int a = 0; a < kAcc / 2; ++a) acc[a][j] += acc[a + kAcc / 2][j];
+      sum[j] = kAcc == 2 ? acc[0][j] : acc[0][j] + acc[1 % kAcc][j];
+    }
+    if (live) {
+      const Real f = nrm[li] * nrm_inv[1];
+      w[i] = row_out(sum[0] + rest_r, sum[1] + rest_i, f, (Real)row_ezz(s, facs, P, H), vi);
+    }
+  }
+}
+
 template <bool kTorus>
 __global__ void __launch_bounds__(kHvThreads) k_count_offdiag(SectorView V, unsigned long long* __restrict__ nnz) {
   __shared__ SectorParams P;
@@ -161,14 +302,14 @@ __global__ void __launch_bounds__(kHvThreads) k_count_offdiag(SectorView V, unsi
 }
 
 template <typename K>
-int persistent_grid(K kernel, size_t smem, int64_t rows) {
+int persistent_grid(K kernel, size_t smem, int64_t rows, int threads = kHvThreads) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kHvThreads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
   if (per_sm < 1) per_sm = 1;
-  int64_t want = (rows + kHvThreads - 1) / kHvThreads;
+  int64_t want = (rows + threads - 1) / threads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
 }
 
@@ -182,6 +323,31 @@ cudaError_t launch_t(const Sector& S, const void* v, void* w, cudaStream_t st) {
   return cudaGetLastError();
 }
 
+template <typename Real, int kOrb>
+cudaError_t launch_free(const Sector& S, int orb, const void* v, void* w, cudaStream_t st) {
+  using CT = typename CT2<Real>::T;
+  const size_t at = align16(pass_smem_bytes(S.P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm));
+  const size_t smem = free_smem_bytes<Real>(S, orb);
+  auto kern = k_hv_free<Real, kOrb>;
+  const int grid = persistent_grid(kern, smem, S.P.n_p, kFreeThreads);
+  const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
+  kern<<<grid, kFreeThreads, smem, st>>>(S.V, tab, S.n_vals, (int)at, reinterpret_cast<const CT*>(v),
+                                         reinterpret_cast<CT*>(w));
+  return cudaGetLastError();
+}
+
+template <typename Real>
+cudaError_t launch_free_t(const Sector& S, const void* v, void* w, cudaStream_t st) {
+  const int orb = orb_of(S.P);
+  switch (orb) {
+    case kOrbPacked: return launch_free<Real, kOrbPacked>(S, orb, v, w, st);
+    case kOrbPacked32: return launch_free<Real, kOrbPacked32>(S, orb, v, w, st);
+    case kOrbPacked64: return launch_free<Real, kOrbPacked64>(S, orb, v, w, st);
+    case kOrbTorus: return launch_free<Real, kOrbTorus>(S, orb, v, w, st);
+    default: return launch_free<Real, kOrbWalk>(S, orb, v, w, st);
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_hv(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st) {
@@ -191,6 +357,9 @@ cudaError_t launch_hv(const Sector& S, const void* v, void* w, bool fp64, cudaSt
 
 cudaError_t launch_hv_generic(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st) {
   const bool torus = S.P.torus != 0, chch = S.P.use_chch != 0;
+  // the table beside the queues in shared memory: up to 2,048 FP64 values
+  if (!chch && S.n_vals > 0 && S.n_vals <= 2048)
+    return fp64 ? launch_free_t<double>(S, v, w, st) : launch_free_t<float>(S, v, w, st);
   if (fp64) {
     if (torus) return chch ? launch_t<double, true, true>(S, v, w, st) : launch_t<double, true, false>(S, v, w, st);
     return chch ? launch_t<double, false, true>(S, v, w, st) : launch_t<double, false, false>(S, v, w, st);

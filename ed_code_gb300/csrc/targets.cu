@@ -36,114 +36,14 @@
 #include "csr_row.cuh"
 #include "hv_common.cuh"
 #include "hv_rows.cuh"
+#include "row_walk.cuh"
 
 namespace edg {
 
 namespace {
 
 constexpr int kPassThreads = 128;
-constexpr int kMaxRowSlots = 256;  // a row has at most one entry per flip group
 constexpr int kMaxChPerGroup = 4;
-
-// A flip group as the passes below stage it: what a row needs to find out
-// whether the pair is anti-aligned, and where its sites sit on a packed torus.
-struct PassGroup {
-  uint64_t mask;
-  uint64_t facadd;        // 1 << 16 * fid: counts the row's anti-aligned pairs by diagonal part
-  double fac;
-  uint16_t off;           // first value variant
-  int16_t a, ch_begin, ch_end;
-  int8_t sa, sb, ba, bb;  // packed torus: bit offset of each site's row in the state, of its byte
-  int8_t top, pad[3];     // packed torus: the pair touches the top row
-};
-
-// Which orbit search the passes use: the reference's walk, the row-rotation
-// search, or the row-rotation search on packed rows (row length and row count
-// up to 8) with 32-bit states and minima, 32-bit states, or 64-bit ones.
-constexpr int kOrbWalk = 0, kOrbTorus = 1, kOrbPacked = 2, kOrbPacked32 = 3, kOrbPacked64 = 4;
-template <int kOrb>
-struct OrbRows {
-  using T = PackedRows<uint64_t, uint64_t>;
-};
-template <>
-struct OrbRows<kOrbPacked> {
-  using T = PackedRows<uint32_t, uint32_t>;
-};
-template <>
-struct OrbRows<kOrbPacked32> {
-  using T = PackedRows<uint32_t, uint64_t>;
-};
-int orb_of(const SectorParams& P) {
-  if (!P.torus) return kOrbWalk;
-  if (P.L1 > 8 || P.L2 > 8) return kOrbTorus;
-  return P.n_sites > 32 ? kOrbPacked64 : P.L2 <= 4 ? kOrbPacked : kOrbPacked32;
-}
-
-struct PassSmem {
-  PassGroup* groups;
-  int8_t* z;  // chirality sites
-  const uint8_t* nk;
-  const uint16_t* rots;
-  const uint64_t *p1, *p2, *p3;
-};
-
-size_t pass_smem_bytes(const SectorParams& P, int orb, int row_bits, int n_chunks, int n_perm) {
-  size_t b = align16(sizeof(PassGroup) * P.n_groups) + align16(P.n_ch);
-  if (orb == kOrbWalk) return b + (size_t)n_perm * n_chunks * 256 * sizeof(uint64_t);
-  return b + align16((size_t)3 << row_bits);
-}
-
-template <int kOrb>
-__device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, const uint16_t* voff,
-                               const uint16_t* order, uint8_t* sm) {
-  PassSmem H{};
-  size_t off = 0;
-  H.groups = reinterpret_cast<PassGroup*>(sm);
-  off += align16(sizeof(PassGroup) * P.n_groups);
-  H.z = reinterpret_cast<int8_t*>(sm + off);
-  off += align16(P.n_ch);
-  for (int at = threadIdx.x; at < P.n_groups; at += blockDim.x) {
-    const int g = order[at];
-    const TermGroup src = V.groups[g];
-    PassGroup d{};
-    d.mask = src.mask;
-    d.facadd = P.n_facs <= kMaxFacs ? 1ull << (16 * src.fid) : 0;
-    d.fac = src.fac;
-    d.off = voff[g];
-    d.a = (int16_t)src.a;
-    d.ch_begin = (int16_t)src.ch_begin;
-    d.ch_end = (int16_t)src.ch_end;
-    if (kOrb >= kOrbPacked) {
-      const int ya = src.a / P.L1, yb = src.b / P.L1;
-      d.sa = (int8_t)(P.L1 * ya);
-      d.sb = (int8_t)(P.L1 * yb);
-      d.ba = (int8_t)(8 * ya);
-      d.bb = (int8_t)(8 * yb);
-      d.top = ya == P.L2 - 1 || yb == P.L2 - 1;
-    }
-    H.groups[at] = d;
-  }
-  for (int m = threadIdx.x; m < P.n_ch; m += blockDim.x) H.z[m] = (int8_t)V.ch[m].z;
-  if (kOrb == kOrbWalk) {
-    const int n = V.n_perm * V.n_chunks * 256;
-    uint64_t* p = reinterpret_cast<uint64_t*>(sm + off);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) p[i] = V.perms[i];
-    H.p1 = p;
-    H.p2 = p + V.n_chunks * 256;
-    H.p3 = p + 2 * V.n_chunks * 256;
-  } else {
-    const int n = 1 << V.row_bits;
-    uint16_t* rots = reinterpret_cast<uint16_t*>(sm + off);
-    uint8_t* nk = sm + off + 2 * n;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      rots[i] = V.rots[i];
-      nk[i] = V.nk[i];
-    }
-    H.rots = rots;
-    H.nk = nk;
-  }
-  return H;
-}
 
 // Pass 1 (count) and pass 2 (fill) share this walk over the rows' targets: a
 // thread owns a row and all of them go through the flip groups together, those
@@ -155,8 +55,8 @@ __device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, const
 // addresses.  Counting needs no rank for a target that is alone in its orbit
 // search (one candidate translate): its stabiliser is trivial, so it is
 // allowed.  The fill pass writes each entry's value id as
-// remap[(pair variant) x class], the index into the deduplicated value table,
-// packed above the column when cb > 0 (csr_row.cuh).
+// remap[(pair variant) x class], the index into the deduplicated value table
+// (value_tables), packed above the column when cb > 0 (csr_row.cuh).
 //
 // Both passes are bound by integer issue (ALU pipe 65 %, 17-20 lanes of a warp
 // active), not by memory.  With a warp per row and a lane per pair they took
@@ -164,10 +64,8 @@ __device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, const
 // took 7.9 + 14.1 ms with 64-bit states, and the sector up to its first H v
 // 54 ms, 34 ms, and 29 ms with 32-bit states.
 template <int kOrb, bool kFill>
-__global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const uint16_t* __restrict__ voff,
-                                                           const uint16_t* __restrict__ order,
-                                                           const uint16_t* __restrict__ remap, int cb,
-                                                           uint32_t* __restrict__ counts, double* __restrict__ ezz,
+__global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb, uint32_t* __restrict__ counts,
+                                                           double* __restrict__ ezz,
                                                            const uint64_t* __restrict__ row_ptr,
                                                            uint32_t* __restrict__ col, uint16_t* __restrict__ vid) {
   __shared__ SectorParams P;
@@ -176,26 +74,17 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const u
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
     reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
   __syncthreads();
-  const PassSmem H = stage_pass<kOrb>(V, P, voff, order, sm);
+  const PassSmem H = stage_pass<kOrb>(V, P, sm);
   __syncthreads();
-  using R = typename OrbRows<kOrb>::T;
-  using St = typename R::State;
-  using Kb = typename R::Bytes;
-  const int ng = P.n_groups, Lx = P.L1;
-  const St rmask = ((St)1 << Lx) - 1;
-  const Kb valid = kOrb >= kOrbPacked ? R::valid(P) : 0;
-  const bool count_facs = P.n_facs <= kMaxFacs;
+  using St = typename OrbRows<kOrb>::T::State;
+  const int ng = P.n_groups;
   const int64_t n_p = P.n_p, stride = (int64_t)gridDim.x * blockDim.x;
   for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_p; base += stride) {
     const int64_t i = base + threadIdx.x;
     const bool live = i < n_p;
     const St s = live ? (St)V.reps[i] : 0;  // no pair is anti-aligned past the end
-    Kb kb = 0;
     uint64_t facs = 0, pos = 0;
-    int mstar = 0;
-    bool uniq = false;
     uint32_t cnt = 0;
-    double fac = 0.0;
     uint2* slot = slots[kFill ? threadIdx.x >> 5 : 0];
     if (kFill) {
       // where the slice's slots start, and which rows have them (csr_row.cuh)
@@ -210,73 +99,36 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, const u
       __syncwarp();
       pos = sl.base;
     }
-    if (kOrb >= kOrbPacked) {
-      // s is a representative: its top row is at its rotation minimum and no
-      // row has a smaller one.  When it is the only row that reaches it and is
-      // aperiodic, a flip that leaves it alone and gives no other row a
-      // minimum <= mstar is its own representative with stabiliser 1.
-      kb = R::pack(s, P, H.nk);
-      Kb hit;
-      mstar = R::min_rows(kb, valid, hit);
-      uniq = R::single(hit) && H.rots[(int)((s >> (Lx * (P.L2 - 1))) & rmask)] == 1u;
-    }
+    RowStart<kOrb> row;
+    row.set(s, P, H);
     for (int g = 0; g < ng; ++g) {
       const PassGroup& gr = H.groups[g];
       const St pm = (St)gr.mask, both = s & pm;
       const bool anti = both != 0 && both != pm;
       if (!__any_sync(0xffffffffu, anti)) continue;
       if (!anti) continue;
-      if (!kFill) {
-        facs += gr.facadd;
-        if (!count_facs) fac += gr.fac;
-      }
-      const St t = s ^ pm;
-      Orbit o;
-      bool known = false;  // allowed for certain (counting)
-      if (kOrb >= kOrbPacked) {
-        const int na = H.nk[(int)((t >> gr.sa) & rmask)], nb = H.nk[(int)((t >> gr.sb) & rmask)];
-        if (uniq && !gr.top && na > mstar && nb > mstar) {
-          o = Orbit{(uint64_t)t, 0, 1};
-          known = true;
-        } else {
-          Kb hit;
-          R::min_rows(R::set(R::set(kb, gr.ba, na), gr.bb, nb), valid, hit);
-          if (!kFill && R::single(hit)) {
-            const uint32_t rs = H.rots[(int)((t >> (Lx * R::row_of(hit))) & rmask)];
-            known = (rs & (rs - 1)) == 0;
-          }
-          if (kFill || !known) o = R::search(t, hit, P, H.rots);
-        }
-      } else if (kOrb == kOrbTorus) {
-        o = orbit_torus(t, P, H.nk, H.rots);
-      } else {
-        o = orbit_walk(t, P, H.p1, H.p2, H.p3, V.n_chunks);
-      }
+      if (!kFill) facs += gr.facadd;
+      bool known;
+      const Orbit o = target_orbit<kOrb, !kFill>((St)(s ^ pm), gr, row, P, H, V.n_chunks, known);
       if (!kFill) {
         if (known || position(o, V, P) >= 0) ++cnt;
+        continue;
+      }
+      const int64_t j = position(o, V, P);
+      if (j < 0) continue;
+      const uint32_t id = value_id(s, gr, o.g, V, P, H);
+      const uint2 sk = slot[cnt++];
+      const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
+      if (cb) {
+        col[p] = (uint32_t)j | (id << cb);
       } else {
-        const int64_t j = position(o, V, P);
-        if (j >= 0) {
-          int variant = (int)((s >> gr.a) & 1u);
-          for (int m = gr.ch_begin, b = 1; m < gr.ch_end; ++m, ++b) variant |= (int)((s >> H.z[m]) & 1u) << b;
-          const uint32_t id = __ldg(remap + (gr.off + variant) * P.n_cls + P.g2cls[o.g]);
-          const uint2 sk = slot[cnt++];
-          const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
-          if (cb) {
-            col[p] = (uint32_t)j | (id << cb);
-          } else {
-            col[p] = (uint32_t)j;
-            vid[p] = (uint16_t)id;
-          }
-        }
+        col[p] = (uint32_t)j;
+        vid[p] = (uint16_t)id;
       }
     }
     if (!kFill && live) {
-      if (count_facs) {
-        for (int k = 0; k < P.n_facs; ++k) fac += P.facs[k] * (double)((facs >> (16 * k)) & 0xFFFFu);
-      }
       counts[i] = cnt;
-      ezz[i] = P.total_fac - 2.0 * fac;  // Ezz = sum_bonds lJ/4 - 2 sum_anti lJ/4
+      ezz[i] = row_ezz(s, facs, P, H);
     }
   }
 }
@@ -471,7 +323,7 @@ int64_t gcd64(int64_t a, int64_t b) {
 }  // namespace
 
 void free_targets(Sector& S) {
-  void* ptrs[] = {S.row_ptr, S.col, S.vid, S.ezz, S.vtab64, S.vtab32, S.ubuf.ptr};
+  void* ptrs[] = {S.row_ptr, S.col, S.vid, S.ezz, S.ubuf.ptr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   S.row_ptr = nullptr;
@@ -479,33 +331,22 @@ void free_targets(Sector& S) {
   S.vid = nullptr;
   S.pack_cb = 0;
   S.ezz = nullptr;
-  S.vtab64 = nullptr;
-  S.vtab32 = nullptr;
-  S.n_vals = 0;
   S.ubuf = DeviceBuffer{};
   S.P.n_targets = 0;
   S.device_bytes -= S.targets_bytes;
   S.targets_bytes = 0;
 }
 
-// Returns EDG_OK, or a reason (EDG_ERR_NOMEM / EDG_ERR_UNSUPPORTED) with the
-// sector left on the matrix-free kernels.
-int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
-  SectorParams& P = S.P;
-  if (S.col) return EDG_OK;
-  if (P.use_chch) {
-    err = "stored targets do not cover ChCh terms";
-    return EDG_ERR_UNSUPPORTED;
-  }
+// Value tables of a sector: for every flip group and variant (bit a of the
+// state, the bits z of its chirality terms) and phase class of a translation,
+// the id of coefficient x phase among the distinct values (compared by bits;
+// with uniform couplings a handful).  Sets P.n_cls and P.g2cls.
+int value_tables(SectorParams& P, const std::vector<TermGroup>& groups, const std::vector<ChTerm>& ch,
+                 ValueTables& T) {
   if (P.n_groups > kMaxRowSlots) {
-    err = "stored targets need at most 256 flip groups";
+    T.why = "stored targets need at most 256 flip groups";
     return EDG_ERR_UNSUPPORTED;
   }
-  // host copies of the term groups (for the value table)
-  std::vector<TermGroup> groups(P.n_groups);
-  std::vector<ChTerm> ch(P.n_ch);
-  cudaMemcpy(groups.data(), S.groups, sizeof(TermGroup) * groups.size(), cudaMemcpyDeviceToHost);
-  if (!ch.empty()) cudaMemcpy(ch.data(), S.ch, sizeof(ChTerm) * ch.size(), cudaMemcpyDeviceToHost);
   // phase classes: translation (a, b, c) has phase index
   // (kx a L2 L3 + ky b L1 L3 + kz c L1 L2) mod G, G = L1 L2 L3 (c = 0 in 2-D)
   const int G = P.L1 * P.L2 * P.L3;
@@ -528,14 +369,12 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
         }
       }
   P.n_cls = n_cls;
-  // value table: for each group, every (bit a, chirality z bits) variant
-  std::vector<uint16_t> voff(P.n_groups);
-  std::vector<double2> tab64;
   int64_t n_var = 0;
+  std::vector<uint16_t> voff(P.n_groups);
   for (int g = 0; g < P.n_groups; ++g) {
     const int nch = groups[g].ch_end - groups[g].ch_begin;
     if (nch > kMaxChPerGroup) {
-      err = "stored targets: more than 4 chirality terms on one pair";
+      T.why = "stored targets: more than 4 chirality terms on one pair";
       return EDG_ERR_UNSUPPORTED;
     }
     if (n_var > 65535) break;
@@ -543,10 +382,22 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     n_var += 2 << nch;
   }
   if (n_var * n_cls > 65536) {
-    err = "stored targets: more than 65536 distinct values";
+    T.why = "stored targets: more than 65536 distinct values";
     return EDG_ERR_UNSUPPORTED;
   }
-  tab64.resize(n_var * n_cls);
+  // distinct coefficients first, then their products with the phases
+  using Key = std::pair<uint64_t, uint64_t>;
+  auto key_of = [](std::complex<double> z) {
+    const double re = z.real(), im = z.imag();
+    Key k;
+    std::memcpy(&k.first, &re, 8);
+    std::memcpy(&k.second, &im, 8);
+    return k;
+  };
+  std::map<Key, int> coefs;
+  std::map<Key, uint16_t> values;
+  std::vector<std::vector<uint16_t>> ids;  // of a coefficient, by class
+  T.remap.resize(n_var * n_cls);
   for (int g = 0; g < P.n_groups; ++g) {
     const TermGroup& gr = groups[g];
     const int nch = gr.ch_end - gr.ch_begin;
@@ -558,84 +409,73 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
         const double sg = ((variant >> (q + 1)) & 1) ? 1.0 : -1.0;
         c += sg * std::complex<double>(t.Are[cs], t.Aim[cs]);
       }
-      for (int cl = 0; cl < n_cls; ++cl) {
-        const std::complex<double> val = c * cph[cl];
-        tab64[(voff[g] + variant) * n_cls + cl] = make_double2(val.real(), val.imag());
+      const auto at = coefs.emplace(key_of(c), (int)ids.size());
+      if (at.second) {
+        ids.emplace_back(n_cls);
+        for (int cl = 0; cl < n_cls; ++cl) {
+          const std::complex<double> val = c * cph[cl];
+          const auto v = values.emplace(key_of(val), (uint16_t)T.v64.size());
+          if (v.second) {
+            T.v64.push_back(make_double2(val.real(), val.imag()));
+            T.v32.push_back(make_float2((float)val.real(), (float)val.imag()));
+          }
+          ids.back()[cl] = v.first->second;
+        }
       }
+      std::copy(ids[at.first->second].begin(), ids[at.first->second].end(),
+                T.remap.begin() + (size_t)(voff[g] + variant) * n_cls);
     }
   }
-  // Deduplicate the table by bit pattern: with uniform couplings many
-  // (pair, variant, class) combinations share one value.  remap[k] is the
-  // index of combination k in the deduplicated table.
-  std::vector<uint16_t> remap(tab64.size());
-  {
-    std::map<std::pair<uint64_t, uint64_t>, uint16_t> index;
-    std::vector<double2> uniq;
-    for (size_t k = 0; k < tab64.size(); ++k) {
-      std::pair<uint64_t, uint64_t> key;
-      std::memcpy(&key.first, &tab64[k].x, 8);
-      std::memcpy(&key.second, &tab64[k].y, 8);
-      auto it = index.find(key);
-      if (it == index.end()) {
-        it = index.emplace(key, (uint16_t)uniq.size()).first;
-        uniq.push_back(tab64[k]);
-      }
-      remap[k] = it->second;
-    }
-    tab64.swap(uniq);
+  // The rows take the groups of high sites first: consecutive representatives
+  // differ in their low sites, so a pair of high sites is anti-aligned in all
+  // rows of a warp or in none, and its targets in neighbouring rows are
+  // neighbours.
+  std::vector<uint16_t> order(P.n_groups);
+  for (int g = 0; g < P.n_groups; ++g) order[g] = (uint16_t)g;
+  std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
+    return groups[p].a != groups[q].a ? groups[p].a > groups[q].a : groups[p].b > groups[q].b;
+  });
+  T.voff.swap(voff);
+  T.order.swap(order);
+  return EDG_OK;
+}
+
+// Returns EDG_OK, or a reason (EDG_ERR_NOMEM / EDG_ERR_UNSUPPORTED) with the
+// sector left on the matrix-free kernels.
+int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
+  SectorParams& P = S.P;
+  if (S.col) return EDG_OK;
+  if (P.use_chch) {
+    err = "stored targets do not cover ChCh terms";
+    return EDG_ERR_UNSUPPORTED;
   }
-  std::vector<float2> tab32(tab64.size());
-  for (size_t k = 0; k < tab64.size(); ++k) tab32[k] = make_float2((float)tab64[k].x, (float)tab64[k].y);
+  if (!S.n_vals) {
+    err = S.values_err;
+    return EDG_ERR_UNSUPPORTED;
+  }
   // Packed entries when the value ids and the columns fit one u32 together:
   // vb bits of value id above cb = 32 - vb column bits, n_p < 2^cb.
   // EDG_ROW_FORMAT=split keeps the two arrays (for comparisons).
   int vb = 1;
-  while ((size_t(1) << vb) < tab64.size()) ++vb;
+  while ((1 << vb) < S.n_vals) ++vb;
   const char* fmt_env = std::getenv("EDG_ROW_FORMAT");
   const bool want_split = fmt_env && std::strcmp(fmt_env, "split") == 0;
   const int cb = 32 - vb;
   S.pack_cb = (!want_split && vb < 32 && P.n_p < (int64_t(1) << cb)) ? cb : 0;
   const double entry_bytes = S.pack_cb ? 4.0 : 6.0;
 
-  // The passes take the groups of high sites first: consecutive representatives
-  // differ in their low sites, so a pair of high sites is anti-aligned in all
-  // rows of a warp or in none, and its targets in neighbouring rows are
-  // neighbours.
-  {
-    std::vector<uint16_t> order(P.n_groups);
-    for (int g = 0; g < P.n_groups; ++g) order[g] = (uint16_t)g;
-    std::stable_sort(order.begin(), order.end(), [&](int p, int q) {
-      return groups[p].a != groups[q].a ? groups[p].a > groups[q].a : groups[p].b > groups[q].b;
-    });
-    voff.insert(voff.end(), order.begin(), order.end());
-  }
-
   cudaStream_t st = S.stream;
   const int64_t n = P.n_p;
   uint32_t* counts = nullptr;
-  uint16_t *d_voff = nullptr, *d_remap = nullptr;  // voff, then the groups' order
   unsigned long long *sums = nullptr, *tot = nullptr;
   const int64_t n_chunks = (n + kChunk - 1) / kChunk;
-  cudaError_t e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&counts, sizeof(uint32_t) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&d_voff, sizeof(uint16_t) * voff.size());
-  if (e == cudaSuccess) e = cudaMalloc(&d_remap, sizeof(uint16_t) * remap.size());
-  if (e == cudaSuccess)
-    e = cudaMemcpy(d_remap, remap.data(), sizeof(uint16_t) * remap.size(), cudaMemcpyHostToDevice);
+  cudaError_t e = cudaMalloc(&counts, sizeof(uint32_t) * n);
   if (e == cudaSuccess) e = cudaMalloc(&sums, sizeof(unsigned long long) * n_chunks);
   if (e == cudaSuccess) e = cudaMalloc(&tot, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc(&S.row_ptr, sizeof(uint64_t) * (n + 1));
   if (e == cudaSuccess) e = cudaMalloc(&S.ezz, sizeof(double) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&S.vtab64, sizeof(double2) * tab64.size());
-  if (e == cudaSuccess) e = cudaMalloc(&S.vtab32, sizeof(float2) * tab32.size());
-  if (e == cudaSuccess) e = cudaMemcpy(d_voff, voff.data(), sizeof(uint16_t) * voff.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(S.vtab64, tab64.data(), sizeof(double2) * tab64.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(S.vtab32, tab32.data(), sizeof(float2) * tab32.size(), cudaMemcpyHostToDevice);
-  S.n_vals = (int)tab64.size();
   auto cleanup = [&]() {
     cudaFree(counts);
-    cudaFree(d_voff);
-    cudaFree(d_remap);
     cudaFree(sums);
     cudaFree(tot);
   };
@@ -649,7 +489,7 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   const size_t smem = pass_smem_bytes(P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm);
   auto pass = [&](auto kern) {
     kern<<<grid_for(kern, smem, n, kPassThreads), kPassThreads, smem, st>>>(
-        S.V, d_voff, d_voff + P.n_groups, d_remap, S.pack_cb, counts, S.ezz, S.row_ptr, S.col, S.vid);
+        S.V, S.pack_cb, counts, S.ezz, S.row_ptr, S.col, S.vid);
   };
   if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, false>);
   else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, false>);
@@ -695,7 +535,7 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     return EDG_ERR_CUDA;
   }
   P.n_targets = (int64_t)nnz;
-  S.targets_bytes = (S.pack_cb ? 4 : 6) * nnz + 8 * (n + 1) + 8 * n + 16 * n + 24 * tab64.size();
+  S.targets_bytes = (S.pack_cb ? 4 : 6) * nnz + 8 * (n + 1) + 8 * n + 16 * n;
   S.device_bytes += S.targets_bytes;
   e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? EDG_OK : EDG_ERR_CUDA;

@@ -68,3 +68,34 @@ def test_row_sums_of_every_split_match_oracle(cuda_device, Lx, Ly, Sz, k):
         torch.cuda.synchronize()
         for q in range(4):
             assert np.array_equal(W.cpu().numpy()[:, q], one), (dt, q)
+
+
+@pytest.mark.parametrize("Lx,Ly,Sz,k,J2,directions", [
+    (4, 3, 0, (0, 0), 0.0, False),     # 75 rows at k = 0: many stabilisers, a part of a slice
+    (8, 4, 11, (0, 2), 0.0, False),    # 32-bit states, stabilisers beside general targets
+    (6, 5, 10, (3, 0), 0.4, True),     # more diagonal parts than are counted
+    (8, 5, -16, (4, 0), 0.0, False),   # 64-bit states
+    (9, 4, -14, (0, 0), 0.0, False),   # the general row-rotation search
+    (6, 4, 0, (3, 2), 0.3, True),      # 112,632 rows, queues of more than one turn
+])
+def test_matrix_free_of_every_search_matches_oracle(cuda_device, Lx, Ly, Sz, k, J2, directions):
+    """The matrix-free H*v and the stored rows against the oracle (FP64 1e-13,
+    FP32 2e-5), also with another coupling in every bond direction."""
+    from ed_code_gb300 import lattice as L
+    from ed_code_gb300 import sector
+
+    model = L.make_model(L.TorusSpec("triangular", Lx, Ly, Jz=0.7, J2=J2, Ch=0.3), Sz, *k, bowties=False)
+    if directions:
+        for b in model.adj_list:
+            d = ((b.y - b.x) % Lx, (b.y // Lx - b.x // Lx) % Ly)
+            b.J *= 1.0 + 0.1 * min(d, ((-d[0]) % Lx, (-d[1]) % Ly))[0] + 0.07 * d[1] * (Ly - d[1])
+    ref = O.OracleSector(model)
+    sec = sector.GpuSector(model)
+    v = O.splitmix_vector(sec.n_p, 8)
+    w = ref.hv(v)
+    scale = max(1.0, np.abs(w).max())
+    for stored in (False, True):
+        if stored:
+            assert sec.build_targets()
+        for dt, tol in ((np.complex128, 1e-13), (np.complex64, 2e-5)):
+            assert np.abs(sec.sHv(v.astype(dt), dtype=dt) - w).max() / scale <= tol, (stored, dt)
