@@ -12,15 +12,12 @@
 //      Hermitian matrices: H_k = I - tau_k v_k v_k^H with a complex tau_k
 //      that makes the sub-diagonal real).  Step k: the reflector of column k,
 //      p = tau A22 v, w = p - (tau/2)(p^H v) v, and the rank-2 update
-//      A22 -= v w^H + w v^H, four kernels.
-//   3. All n eigenvalues of T, one thread each: bisection on FP32 Sturm
-//      counts to about 1e-7 of |T|, then Newton's method on det(T - x I) in
-//      FP64 (three-term recurrence for the determinant and its derivative,
-//      rescaled by powers of two), checked with FP64 Sturm counts at
-//      x -+ 4 eps |T|; an eigenvalue that fails the check (a multiple or a
-//      tightly clustered root) is bisected in FP64 instead.  Bisection on all
-//      n eigenvalues in FP64 alone would take ~50 n FP64 passes per
-//      eigenvalue, and GB300 runs FP64 at 1/64 of its FP32 rate.
+//      A22 -= v w^H + w v^H, in two kernels on the lower triangle: one brings
+//      column k up to date and takes its reflector, the other applies the
+//      previous step's update and multiplies by the new v in one pass.
+//   3. All n eigenvalues of T, eight lanes each: multisection on Sturm counts
+//      (the signs of the leading minors) in FP32 to about 1e-7 of |T|, then in
+//      FP64 from there; GB300 runs FP64 at 1/64 of its FP32 rate.
 //   4. The wanted eigenvectors: inverse iteration on T (tridiag.cuh;
 //      orthogonalised within clusters of equal eigenvalues), then x = Q y by
 //      applying the reflectors from the last to the first.
@@ -114,182 +111,339 @@ __device__ double block_sum(double x, double* sh) {
   return r;
 }
 
-// Step k, part 1 (one CTA): the reflector of column k below the diagonal,
-// x = A[k+1.., k] -> v = (1, x_1/(alpha - beta), ...), stored in place;
-// d[k], e[k] = beta, tau[k].
-__global__ void __launch_bounds__(kDenseThreads) k_hh_reflect(double2* __restrict__ A, int64_t n, int64_t k,
-                                                              double* __restrict__ d, double* __restrict__ e,
-                                                              double2* __restrict__ tau) {
-  __shared__ double sh[kDenseThreads];
-  __shared__ double2 inv;
-  __shared__ int apply;
-  const int64_t m = n - k - 1;
-  double2* x = A + k * n + (k + 1);
-  double s = 0.0;
-  for (int64_t i = 1 + threadIdx.x; i < m; i += blockDim.x) s += x[i].x * x[i].x + x[i].y * x[i].y;
-  s = block_sum(s, sh);
+// The reduction's state beside A (n x n, column-major, lower triangle): v_k is
+// stored in column k below the diagonal, as the back-transformation wants it.
+// What a step leaves for the next is kept twice, by the parity of k.
+constexpr int kTile = 32, kTileThreads = 128;
+struct Hh {
+  double2* A;
+  int64_t n;
+  int nb;         // blocks of kTile rows
+  double *d, *e;
+  double2* tau;
+  double2* x;     // [2][n]: column k, up to date, before its scaling: v = x inv, v_{k+1} = 1
+  double2* inv;   // [2]
+  double2* y;     // [2][n]: A22 v
+  double2* D;     // per block of rows: sum conj(y) v
+  double2* K;     // [2]: -|tau|^2/2 v^H A v: w = tau y + K v
+  double2* part;  // nb x n: the tiles' shares of y
+  double* norms;  // the reflector's CTAs' shares of |x|^2
+  int* cnt;       // nb + 1 tickets, zero between launches
+};
+
+// The sum of x over a CTA of kTileThreads, in every thread: shuffles and one
+// round through shared memory.
+__device__ __forceinline__ double tile_sum(double x) {
+  __shared__ double sh[kTileThreads / 32];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+  __syncthreads();
+  double s = sh[0];
+#pragma unroll
+  for (int w = 1; w < kTileThreads / 32; ++w) s += sh[w];
+  return s;
+}
+
+// true in the CTA that takes the last of `total` tickets (no CTA waits)
+__device__ __forceinline__ bool hh_last(int* cnt, int total) {
+  __shared__ int last;
+  __syncthreads();
   if (threadIdx.x == 0) {
-    d[k] = A[k * n + k].x;
-    const double2 alpha = x[0];
-    double2 t = make_double2(0.0, 0.0);
-    double beta = alpha.x;
-    apply = 0;
+    __threadfence();
+    last = atomicAdd(cnt, 1) == total - 1;
+    if (last) *cnt = 0;
+  }
+  __syncthreads();
+  const bool r = last != 0;
+  if (r) __threadfence();
+  __syncthreads();
+  return r;
+}
+
+__device__ __forceinline__ double2 ldcg2(const double2* p) { return __ldcg(p); }
+
+// a - v conj(w_j) - w conj(v_j)
+__device__ __forceinline__ double2 rank2(double2 a, double2 v, double2 w, double2 vj, double2 wj) {
+  a.x = fma(-v.x, wj.x, fma(-v.y, wj.y, fma(-w.x, vj.x, fma(-w.y, vj.y, a.x))));
+  a.y = fma(-v.y, wj.x, fma(v.x, wj.y, fma(-w.y, vj.x, fma(w.x, vj.y, a.y))));
+  return a;
+}
+
+// Step k, first kernel: column k with step k-1's update, x = A[k+1.., k] -> its
+// reflector v = (1, x_1/(alpha - beta), ...): d[k], e[k] = beta, tau[k].  A CTA
+// per 128 rows; the last one finishes the norm and the scalars.
+__global__ void __launch_bounds__(kTileThreads) k_hh_column(Hh H, int64_t k) {
+  const int64_t n = H.n;
+  const int p = (int)(k & 1), lane = threadIdx.x & 31;
+  double2 Kc = make_double2(0.0, 0.0), t = make_double2(0.0, 0.0), wk = Kc;
+  const double2* vo = H.A + (k - 1) * n;  // v_{k-1}: 1 at row k
+  const double2* yo = H.y + (1 - p) * n;
+  if (k > 0) {  // w_{k-1} = t y + K v, K from the blocks' shares in block order
+    __shared__ double2 sK;
+    if (threadIdx.x < 32) {
+      double a = 0, b = 0;
+      for (int r = (int)(k / kTile) + lane; r < H.nb; r += 32) {
+        const double2 q = H.D[r];
+        a += q.x;
+        b += q.y;
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+      }
+      if (lane == 0) {
+        const double2 tt = H.tau[k - 1];
+        const double h = -0.5 * (tt.x * tt.x + tt.y * tt.y);
+        sK = make_double2(h * a, h * b);
+        if (blockIdx.x == 0) H.K[1 - p] = sK;
+      }
+    }
+    __syncthreads();
+    Kc = sK;
+    t = H.tau[k - 1];
+    wk = cmul(t, yo[k]);
+    wk.x += Kc.x;
+    wk.y += Kc.y;
+  }
+  const int64_t i = k + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  double s = 0.0;
+  if (i < n) {
+    double2 a = H.A[k * n + i];
+    if (k > 0) {
+      const double2 v = i == k ? make_double2(1.0, 0.0) : vo[i];
+      double2 w = cmul(t, yo[i]);
+      const double2 kv = cmul(Kc, v);
+      w.x += kv.x;
+      w.y += kv.y;
+      a = rank2(a, v, w, make_double2(1.0, 0.0), wk);
+    }
+    if (i == k) H.d[k] = a.x;
+    else H.x[p * n + i] = a;
+    if (i > k + 1) s = a.x * a.x + a.y * a.y;
+  }
+  if (k + 1 >= n) return;
+  s = tile_sum(s);
+  if (threadIdx.x == 0) H.norms[blockIdx.x] = s;
+  if (!hh_last(H.cnt + H.nb, gridDim.x)) return;
+  s = 0.0;
+  for (int q = threadIdx.x; q < (int)gridDim.x; q += blockDim.x) s += __ldcg(H.norms + q);
+  s = tile_sum(s);
+  if (threadIdx.x < 4) {  // the four quotients side by side: a division is a long chain
+    const double2 alpha = ldcg2(H.x + p * n + k + 1);
+    double beta = alpha.x, quot = threadIdx.x == 2 ? 1.0 : 0.0;
     if (s != 0.0 || alpha.y != 0.0) {
       beta = -copysign(sqrt(alpha.x * alpha.x + alpha.y * alpha.y + s), alpha.x);
-      t = make_double2((beta - alpha.x) / beta, -alpha.y / beta);
       const double zr = alpha.x - beta, zi = alpha.y, z2 = zr * zr + zi * zi;
-      inv = make_double2(zr / z2, -zi / z2);
-      apply = 1;
+      const double num = threadIdx.x == 0 ? beta - alpha.x : threadIdx.x == 1 ? -alpha.y : threadIdx.x == 2 ? zr : -zi;
+      quot = num / (threadIdx.x < 2 ? beta : z2);
     }
-    e[k] = beta;
-    tau[k] = t;
+    double* to = reinterpret_cast<double*>(threadIdx.x < 2 ? H.tau + k : H.inv + p);
+    to[threadIdx.x & 1] = quot;
+    if (threadIdx.x == 0) H.e[k] = beta;
+  }
+}
+
+// Step k, second kernel: A22 (rows and columns > k) with step k-1's update, and
+// y = A22 v_k from its lower triangle: a CTA per 32 x 32 tile on or below the
+// diagonal, a lane per row, eight columns a warp.  An element off the diagonal
+// serves y_i and y_j; the eight columns' shares of y_j over the lanes are closed
+// by an exchange that halves them (16 additions instead of 80).  The tiles'
+// shares are summed in block order by the last tile of each block of rows, with
+// sum conj(y) v.  Bound by FP64 issue (16 clocks a warp instruction): 18
+// instructions an element of half the matrix, where separate update (12) and
+// product (4) kernels took 16 of all of it, and passed over it three times.
+// 2,700 states: the first column took 331 us in four kernels and takes 152 us in
+// two (FP64 pipe 79 % busy while an SM has tiles), the whole spectrum 369 ms and
+// 185 ms.
+__global__ void __launch_bounds__(kTileThreads) k_hh_tile(Hh H, int64_t k, int b0) {
+  __shared__ double2 vn[2][kTile], vo[2][kTile], wo[2][kTile];  // rows' and columns' blocks
+  __shared__ double2 ysum[kTileThreads / 32][kTile];
+  const int64_t n = H.n;
+  const int p = (int)(k & 1), lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  // tile (bi, bj), b0 <= bj <= bi: index = r (r + 1) / 2 + c
+  const int idx = blockIdx.x;
+  int r = (int)((sqrtf(8.f * (float)idx + 1.f) - 1.f) * 0.5f);
+  while ((r + 1) * (r + 2) / 2 <= idx) ++r;
+  while (r * (r + 1) / 2 > idx) --r;
+  const int bi = b0 + r, bj = b0 + idx - r * (r + 1) / 2;
+  const int64_t i = (int64_t)bi * kTile + lane, j0 = (int64_t)bj * kTile + 8 * wid;
+  double2 a[8];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {  // in flight during the vectors' preparation
+    const int64_t j = j0 + q;
+    a[q] = make_double2(0.0, 0.0);
+    if (j > k && i >= j && i < n) a[q] = H.A[j * n + i];
+  }
+  if (threadIdx.x < 2 * kTile) {
+    const int side = threadIdx.x >> 5;
+    const int64_t m = (int64_t)(side ? bj : bi) * kTile + lane;
+    double2 f = make_double2(0.0, 0.0), b = f, c = f;
+    if (m > k && m < n) {
+      f = m == k + 1 ? make_double2(1.0, 0.0) : cmul(H.x[p * n + m], H.inv[p]);
+      if (bi == bj && side == 0) H.A[k * n + m] = f;
+      if (k > 0) {
+        b = H.A[(k - 1) * n + m];
+        c = cmul(H.tau[k - 1], H.y[(1 - p) * n + m]);
+        const double2 kv = cmul(H.K[1 - p], b);
+        c.x += kv.x;
+        c.y += kv.y;
+      }
+    }
+    vn[side][lane] = f;
+    vo[side][lane] = b;
+    wo[side][lane] = c;
   }
   __syncthreads();
-  if (apply)
-    for (int64_t i = 1 + threadIdx.x; i < m; i += blockDim.x) x[i] = cmul(x[i], inv);
+  const double2 vi = vn[0][lane], oi = vo[0][lane], wi = wo[0][lane];
+  double yr = 0.0, yi = 0.0, c[16];
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int64_t j = j0 + q;
+    const int jl = 8 * wid + q;
+    const bool in = j > k && i >= j && i < n;
+    if (k > 0) {
+      a[q] = rank2(a[q], oi, wi, vo[1][jl], wo[1][jl]);
+      if (i == j) a[q].y = 0.0;
+      if (in) H.A[j * n + i] = a[q];
+    }
+    if (!in) a[q] = make_double2(0.0, 0.0);
+    const double2 vj = vn[1][jl];
+    yr = fma(a[q].x, vj.x, fma(-a[q].y, vj.y, yr));
+    yi = fma(a[q].x, vj.y, fma(a[q].y, vj.x, yi));
+    const double2 z = i == j ? make_double2(0.0, 0.0) : a[q];
+    c[2 * q] = fma(z.x, vi.x, z.y * vi.y);
+    c[2 * q + 1] = fma(z.x, vi.y, -(z.y * vi.x));
+  }
+#pragma unroll
+  for (int o = 16, w = 8; o >= 2; o >>= 1, w >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      if (j < w) c[j] = (up ? c[w + j] : c[j]) + __shfl_xor_sync(0xffffffffu, up ? c[j] : c[w + j], o);
+  }
+  c[0] += __shfl_xor_sync(0xffffffffu, c[0], 1);  // value lane >> 1 of the 16
+  ysum[wid][lane] = make_double2(yr, yi);
+  __shared__ double cs[kTile][2];
+  if ((lane & 1) == 0) cs[8 * wid + (lane >> 2)][(lane >> 1) & 1] = c[0];
   __syncthreads();
-  if (threadIdx.x == 0) x[0] = make_double2(1.0, 0.0);
-}
-
-// Step k, part 2: p_i = tau (A22 v)_i = tau sum_j conj(A22[j][i]) v_j, a warp
-// per column i of A22 (A22 is Hermitian, its columns are contiguous)
-__global__ void __launch_bounds__(kDenseThreads) k_hh_p(const double2* __restrict__ A, int64_t n, int64_t k,
-                                                        const double2* __restrict__ tau, double2* __restrict__ p) {
-  const int64_t m = n - k - 1;
-  const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  if (i >= m) return;
-  const double2 t = tau[k];
-  if (t.x == 0.0 && t.y == 0.0) {
-    if (lane == 0) p[i] = make_double2(0.0, 0.0);
-    return;
+  if (wid == 0) {
+    double2 z = ysum[0][lane];
+#pragma unroll
+    for (int q = 1; q < kTileThreads / 32; ++q) {
+      z.x += ysum[q][lane].x;
+      z.y += ysum[q][lane].y;
+    }
+    if (bi == bj) {
+      z.x += cs[lane][0];
+      z.y += cs[lane][1];
+    }
+    if (i < n) H.part[(int64_t)bj * n + i] = z;
+  } else if (wid == 1 && bi != bj) {
+    H.part[(int64_t)bi * n + (int64_t)bj * kTile + lane] = make_double2(cs[lane][0], cs[lane][1]);
   }
-  const double2* ci = A + (k + 1 + i) * n + (k + 1);
-  const double2* v = A + k * n + (k + 1);
-  double sr = 0.0, si = 0.0;
-  for (int64_t j = lane; j < m; j += 32) {
-    const double2 a = ci[j], b = v[j];
-    sr += a.x * b.x + a.y * b.y;
-    si += a.x * b.y - a.y * b.x;
+  // the last tile of a block of rows closes its y
+  for (int side = 0; side < (bi == bj ? 1 : 2); ++side) {
+    const int blk = side ? bj : bi;
+    if (!hh_last(H.cnt + blk, H.nb - b0)) continue;
+    const int64_t row = (int64_t)blk * kTile + lane;
+    double2 z = make_double2(0.0, 0.0);
+    if (row < n)
+      for (int q = b0 + wid; q < H.nb; q += kTileThreads / 32) {
+        const double2 f = ldcg2(H.part + (int64_t)q * n + row);
+        z.x += f.x;
+        z.y += f.y;
+      }
+    __syncthreads();
+    ysum[wid][lane] = z;
+    __syncthreads();
+    if (wid == 0) {
+#pragma unroll
+      for (int q = 1; q < kTileThreads / 32; ++q) {
+        z.x += ysum[q][lane].x;
+        z.y += ysum[q][lane].y;
+      }
+      if (row < n) H.y[p * n + row] = z;
+      double2 g = cconjmul(z, vn[side][lane]);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        g.x += __shfl_down_sync(0xffffffffu, g.x, o);
+        g.y += __shfl_down_sync(0xffffffffu, g.y, o);
+      }
+      if (lane == 0) H.D[blk] = g;
+    }
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    sr += __shfl_down_sync(0xffffffffu, sr, o);
-    si += __shfl_down_sync(0xffffffffu, si, o);
-  }
-  if (lane == 0) p[i] = cmul(t, make_double2(sr, si));
-}
-
-// Step k, part 3 (one CTA): w = p - (tau/2) (p^H v) v
-__global__ void __launch_bounds__(kDenseThreads) k_hh_w(const double2* __restrict__ A, int64_t n, int64_t k,
-                                                        const double2* __restrict__ tau,
-                                                        const double2* __restrict__ p, double2* __restrict__ w) {
-  __shared__ double sh[kDenseThreads];
-  const int64_t m = n - k - 1;
-  const double2* v = A + k * n + (k + 1);
-  double sr = 0.0, si = 0.0;
-  for (int64_t i = threadIdx.x; i < m; i += blockDim.x) {
-    const double2 q = cconjmul(p[i], v[i]);
-    sr += q.x;
-    si += q.y;
-  }
-  sr = block_sum(sr, sh);
-  si = block_sum(si, sh);
-  const double2 t = tau[k];
-  const double2 K = cmul(make_double2(-0.5 * t.x, -0.5 * t.y), make_double2(sr, si));
-  for (int64_t i = threadIdx.x; i < m; i += blockDim.x) {
-    const double2 kv = cmul(K, v[i]);
-    w[i] = make_double2(p[i].x + kv.x, p[i].y + kv.y);
-  }
-}
-
-// Step k, part 4: A22 -= v w^H + w v^H (real diagonal kept)
-__global__ void k_hh_rank2(double2* __restrict__ A, int64_t n, int64_t k, const double2* __restrict__ tau,
-                           const double2* __restrict__ w) {
-  const int64_t m = n - k - 1;
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y;
-  if (i >= m) return;
-  const double2 t = tau[k];
-  if (t.x == 0.0 && t.y == 0.0) return;
-  const double2* v = A + k * n + (k + 1);
-  const double2 vi = v[i], vj = v[j], wi = w[i], wj = w[j];
-  double2& a = A[(k + 1 + j) * n + (k + 1 + i)];
-  // v_i conj(w_j) + w_i conj(v_j)
-  const double2 u1 = cconjmul(wj, vi), u2 = cconjmul(vj, wi);
-  a.x -= u1.x + u2.x;
-  a.y = i == j ? 0.0 : a.y - (u1.y + u2.y);
-}
-
-__global__ void k_last_diag(const double2* __restrict__ A, int64_t n, double* __restrict__ d) {
-  d[n - 1] = A[(n - 1) * n + (n - 1)].x;
 }
 
 // ---- eigenvalues of T: d[0..n-1], off-diagonal e[0..n-2] (row i to i+1) ----
 
-// eigenvalues of T below x, FP32 Sturm count (pivots q_i; a tiny pivot counts as negative)
-__device__ int count32(const float* d, const float* e2, int n, float x, float pivmin) {
-  int c = 0;
-  float q = d[0] - x;
-  if (fabsf(q) < pivmin) q = -pivmin;
-  c += q < 0.f;
-  for (int i = 1; i < n; ++i) {
-    q = d[i] - x - e2[i - 1] / q;
-    if (fabsf(q) < pivmin) q = -pivmin;
-    c += q < 0.f;
+// Counts of eigenvalues below x from the signs of the leading minors
+// p_i = det(T_i - x), p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}: a sign change
+// from p_{i-1} to p_i is an eigenvalue below x (a zero minor counts once
+// whichever sign it is given).  No division, whose FP64 form is a chain of a
+// dozen instructions, and no comparison on the FP64 pipe: the signs and
+// exponents are read as integers, and every four steps the pair is rescaled by a
+// power of two.  A step's chain is one multiply-add.  e2 has no zeros (k_tri_prep).
+__device__ __forceinline__ int count32(const float* __restrict__ d, const float* __restrict__ e2, int n, float x) {
+  float pm = 1.f, p = d[0] - x;
+  int c = (int)(__float_as_uint(p) >> 31);
+  int i = 1;
+  auto step = [&]() {
+    const float pn = fmaf(d[i] - x, p, -(e2[i - 1] * pm));
+    c += (int)((__float_as_uint(pn) ^ __float_as_uint(p)) >> 31);
+    pm = p;
+    p = pn;
+    ++i;
+  };
+  while (i + 4 <= n) {
+    step();
+    step();
+    step();
+    step();
+    const uint32_t ex = max(__float_as_uint(p) & 0x7F800000u, __float_as_uint(pm) & 0x7F800000u);
+    if (ex > (127u + 30u) << 23) {
+      p *= 0x1p-60f;
+      pm *= 0x1p-60f;
+    } else if (ex < (127u - 30u) << 23) {
+      p *= 0x1p60f;
+      pm *= 0x1p60f;
+    }
   }
+  while (i < n) step();
   return c;
 }
 
-// the same count in FP64 from the signs of the leading minors p_i = det(T_i - x),
-// p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}, rescaled by powers of two; a zero
-// minor counts as a sign change (as a tiny negative pivot would)
-__device__ int count64(const double* d, const double* e2, int n, double x) {
-  int c = 0;
+__device__ __forceinline__ uint32_t exp_of(double x) { return (uint32_t)__double2hiint(x) & 0x7FF00000u; }
+
+__device__ __forceinline__ int count64(const double* __restrict__ d, const double* __restrict__ e2, int n, double x) {
   double pm = 1.0, p = d[0] - x;
-  c += p <= 0.0;
-  if (p == 0.0) p = -1e-300;
-  for (int i = 1; i < n; ++i) {
-    double pn = (d[i] - x) * p - e2[i - 1] * pm;
-    if (pn == 0.0) pn = p > 0 ? -1e-300 * fabs(p) : 1e-300 * fabs(p);
-    c += (pn < 0.0) != (p < 0.0);
+  int c = (int)((uint32_t)__double2hiint(p) >> 31);
+  int i = 1;
+  auto step = [&]() {
+    const double pn = fma(d[i] - x, p, -(e2[i - 1] * pm));
+    c += (int)((uint32_t)(__double2hiint(pn) ^ __double2hiint(p)) >> 31);
     pm = p;
     p = pn;
-    const double ap = fabs(p);
-    if (ap > 0x1p500) {
-      p *= 0x1p-500;
-      pm *= 0x1p-500;
-    } else if (ap < 0x1p-500 && fabs(pm) < 0x1p-500) {
-      p *= 0x1p500;
-      pm *= 0x1p500;
+    ++i;
+  };
+  while (i + 4 <= n) {
+    step();
+    step();
+    step();
+    step();
+    const uint32_t ex = max(exp_of(p), exp_of(pm));
+    if (ex > (1023u + 300u) << 20) {
+      p *= 0x1p-600;
+      pm *= 0x1p-600;
+    } else if (ex < (1023u - 300u) << 20) {
+      p *= 0x1p600;
+      pm *= 0x1p600;
     }
   }
+  while (i < n) step();
   return c;
-}
-
-// one Newton step on det(T - x): returns det / det' (rescaled consistently)
-__device__ double newton_step(const double* d, const double* e2, int n, double x) {
-  double pm = 1.0, p = d[0] - x, dpm = 0.0, dp = -1.0;
-  for (int i = 1; i < n; ++i) {
-    const double a = d[i] - x;
-    const double pn = a * p - e2[i - 1] * pm;
-    const double dpn = a * dp - p - e2[i - 1] * dpm;
-    pm = p;
-    p = pn;
-    dpm = dp;
-    dp = dpn;
-    const double big = fmax(fabs(p), fabs(dp));
-    if (big > 0x1p500) {
-      p *= 0x1p-500;
-      pm *= 0x1p-500;
-      dp *= 0x1p-500;
-      dpm *= 0x1p-500;
-    } else if (big < 0x1p-500 && fmax(fabs(pm), fabs(dpm)) < 0x1p-500) {
-      p *= 0x1p500;
-      pm *= 0x1p500;
-      dp *= 0x1p500;
-      dpm *= 0x1p500;
-    }
-  }
-  return p / dp;
 }
 
 __global__ void k_tri_prep(const double* __restrict__ d, const double* __restrict__ e, int n, float* __restrict__ d32,
@@ -297,58 +451,65 @@ __global__ void k_tri_prep(const double* __restrict__ d, const double* __restric
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     d32[i] = (float)d[i];
     if (i + 1 < n) {
-      e2[i] = e[i] * e[i];
-      e232[i] = (float)e[i] * (float)e[i];
+      // a decoupled row couples by less than any rounding instead (1e-290 and
+      // 1e-30 of |T|^2 ~ 1), so that no minor stays zero
+      e2[i] = fmax(e[i] * e[i], 1e-290);
+      e232[i] = fmaxf((float)e[i] * (float)e[i], 1e-30f);
     }
   }
 }
 
-// eigenvalue k of T, one thread each; bounds [gl, gu] enclose the spectrum
-__global__ void k_tri_all(const double* __restrict__ d, const double* __restrict__ e2, const float* __restrict__ d32,
-                          const float* __restrict__ e232, int n, double gl, double gu, double tnorm,
-                          double* __restrict__ out, int* __restrict__ n_fallback) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= n) return;
-  const float pivf = 1e-30f;
+// One round of multisection for eigenvalue k in (lo, hi] by a group of eight
+// lanes: the counts at eight interior points, and the ninth of the bracket that
+// holds it.  All lanes of the warp take part.
+template <typename R, class Count>
+__device__ __forceinline__ void narrow(R& lo, R& hi, int k, bool run, Count count) {
+  const int sub = threadIdx.x & 7, at = threadIdx.x & 24;
+  const R x = lo + (hi - lo) * ((R)(sub + 1) / (R)9);
+  const unsigned above = (__ballot_sync(0xffffffffu, count(x) > k) >> at) & 0xFFu;
+  const int first = above ? __ffs((int)above) - 1 : 8;  // counts grow with x
+  const R a = __shfl_sync(0xffffffffu, x, at + (first > 0 ? first - 1 : 0));
+  const R b = __shfl_sync(0xffffffffu, x, at + (first < 8 ? first : 7));
+  if (!run) return;
+  if (first > 0) lo = a;
+  if (first < 8) hi = b;
+}
+
+// Eigenvalue k of T by a group of eight lanes; bounds [gl, gu] enclose the
+// spectrum.  FP32 counts to about 1e-7 of |T|, then FP64 counts from a bracket
+// widened by four times that (checked; the whole range if the eigenvalue is not
+// in it) to half an ulp of |T|: ten rounds of three FP64 instructions a row of
+// T, four warps an SM.  Newton's method on the determinant took six passes of
+// twice the instructions and left multiple roots to 31 bisections by one lane,
+// which made it 43 ms at 2,700 states; this takes 5.8 ms.
+__global__ void __launch_bounds__(32) k_tri_all(const double* __restrict__ d, const double* __restrict__ e2,
+                                                const float* __restrict__ d32, const float* __restrict__ e232, int n,
+                                                double gl, double gu, double tnorm, double* __restrict__ out) {
+  const int k = min(n - 1, (int)((blockIdx.x * 32 + threadIdx.x) >> 3));
+  auto c32 = [&](float x) { return count32(d32, e232, n, x); };
+  auto c64 = [&](double x) { return count64(d, e2, n, x); };
   float lo = (float)gl, hi = (float)gu;
-  for (int it = 0; it < 64; ++it) {
-    const float mid = 0.5f * (lo + hi);
-    if (!(mid > lo && mid < hi)) break;
-    if (hi - lo <= 4.f * 1.1920929e-7f * fmaxf(fabsf(lo), fabsf(hi))) break;
-    if (count32(d32, e232, n, mid, pivf) > k) hi = mid;
-    else lo = mid;
+  for (int it = 0; it < 16; ++it) {
+    const bool run = hi - lo > 4.f * 1.1920929e-7f * fmaxf(fabsf(lo), fabsf(hi));
+    if (!__any_sync(0xffffffffu, run)) break;
+    narrow(lo, hi, k, run, c32);
   }
   const double width = (double)hi - (double)lo + 4e-7 * tnorm;
-  double x = 0.5 * ((double)lo + (double)hi);
-  bool ok = true;
-  for (int it = 0; it < 6; ++it) {
-    const double s = newton_step(d, e2, n, x);
-    if (!isfinite(s) || fabs(s) > width) {
-      ok = false;
-      break;
-    }
-    x -= s;
-    if (fabs(s) <= 2.2e-16 * fmax(fabs(x), 1e-300)) break;
+  double a = (double)lo - width, b = (double)hi + width;
+  // lane 0 of a group looks at a, the others at b
+  const int sub = threadIdx.x & 7;
+  const bool below = c64(sub == 0 ? a : b) <= k;
+  const unsigned m = __ballot_sync(0xffffffffu, below) >> (threadIdx.x & 24);
+  if (!(m & 1u)) a = gl;
+  if (m & 2u) b = gu;
+  const double tol = 1.110223024625157e-16 * tnorm;
+  for (int it = 0; it < 24; ++it) {
+    const double x = a + (b - a) * (1.0 / 9.0);
+    const bool run = b - a > tol && x > a && x < b;
+    if (!__any_sync(0xffffffffu, run)) break;
+    narrow(a, b, k, run, c64);
   }
-  const double delta = 4.0 * 2.220446049250313e-16 * fmax(fabs(x), tnorm);
-  if (ok) ok = count64(d, e2, n, x - delta) <= k && count64(d, e2, n, x + delta) > k;
-  if (!ok) {
-    atomicAdd(n_fallback, 1);
-    double a = (double)lo - width, b = (double)hi + width;
-    if (!(count64(d, e2, n, a) <= k && count64(d, e2, n, b) > k)) {
-      a = gl;
-      b = gu;
-    }
-    for (int it = 0; it < 200; ++it) {
-      const double mid = 0.5 * (a + b);
-      if (!(mid > a && mid < b)) break;
-      if (b - a <= 2.0 * 2.220446049250313e-16 * fmax(fabs(a), fabs(b))) break;
-      if (count64(d, e2, n, mid) > k) b = mid;
-      else a = mid;
-    }
-    x = 0.5 * (a + b);
-  }
-  out[k] = x;
+  if (sub == 0) out[k] = 0.5 * (a + b);
 }
 
 // eigenvectors of T for lam[0..nv-1] (ascending), one thread in sequence:
@@ -410,24 +571,28 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
   if (n > 46340) return fail(EDG_ERR_UNSUPPORTED, "dense path: sector too large");
   const int64_t nv = (evecs && evecs_cap > 0) ? std::min<int64_t>(evecs_cap, n) : 0;
   cudaStream_t st = S.stream;
-  double2 *H = nullptr, *tau = nullptr, *pw = nullptr, *X = nullptr;
+  double2 *H = nullptr, *tau = nullptr, *pw = nullptr, *X = nullptr, *part = nullptr;
   double *d = nullptr, *e = nullptr, *e2 = nullptr, *lam = nullptr, *y = nullptr, *wk = nullptr;
   float* f32 = nullptr;
-  int* nfb = nullptr;
+  int* hcnt = nullptr;
+  const int nb = (int)((n + kTile - 1) / kTile);
+  // pw: x, y (two each), D, inv, K, norms
+  const size_t pw_n = (size_t)(4 * n + nb + 4 + (n + kTileThreads) / kTileThreads);
   auto cleanup = [&]() {
-    void* p[] = {H, tau, pw, X, d, e, e2, lam, y, wk, f32, nfb};
+    void* p[] = {H, tau, pw, X, part, hcnt, d, e, e2, lam, y, wk, f32};
     for (void* q : p)
       if (q) cudaFree(q);
   };
   cudaError_t ce = cudaMalloc(&H, sizeof(double2) * n * n);
   if (ce == cudaSuccess) ce = cudaMalloc(&tau, sizeof(double2) * n);
-  if (ce == cudaSuccess) ce = cudaMalloc(&pw, sizeof(double2) * 2 * n);
+  if (ce == cudaSuccess) ce = cudaMalloc(&pw, sizeof(double2) * pw_n);
+  if (ce == cudaSuccess) ce = cudaMalloc(&part, sizeof(double2) * (size_t)nb * n);
+  if (ce == cudaSuccess) ce = cudaMalloc(&hcnt, sizeof(int) * (nb + 1));
   if (ce == cudaSuccess) ce = cudaMalloc(&d, sizeof(double) * n);
   if (ce == cudaSuccess) ce = cudaMalloc(&e, sizeof(double) * n);
   if (ce == cudaSuccess) ce = cudaMalloc(&e2, sizeof(double) * n);
   if (ce == cudaSuccess) ce = cudaMalloc(&lam, sizeof(double) * n);
   if (ce == cudaSuccess) ce = cudaMalloc(&f32, sizeof(float) * 2 * n);
-  if (ce == cudaSuccess) ce = cudaMalloc(&nfb, sizeof(int));
   if (ce == cudaSuccess && nv > 0) ce = cudaMalloc(&X, sizeof(double2) * n * nv);
   if (ce == cudaSuccess && nv > 0) ce = cudaMalloc(&y, sizeof(double) * n * nv);
   if (ce == cudaSuccess && nv > 0) ce = cudaMalloc(&wk, sizeof(double) * 5 * n);
@@ -439,7 +604,6 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
   const auto t0 = clk::now();
   // 1. H
   cudaMemsetAsync(H, 0, sizeof(double2) * n * n, st);
-  cudaMemsetAsync(nfb, 0, sizeof(int), st);
   int64_t hv_calls = 0;
   if (S.col) {
     const double* nrm = reinterpret_cast<const double*>(reinterpret_cast<const char*>(S.dP) +
@@ -463,14 +627,19 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
   const auto t1 = clk::now();
   // 2. Householder tridiagonalisation
   k_herm_upper<<<dim3((unsigned)((n + 255) / 256), (unsigned)n), 256, 0, st>>>(H, n);
-  for (int64_t k = 0; k + 1 < n; ++k) {
-    const int64_t m = n - k - 1;
-    k_hh_reflect<<<1, kDenseThreads, 0, st>>>(H, n, k, d, e, tau);
-    k_hh_p<<<(unsigned)((m * 32 + kDenseThreads - 1) / kDenseThreads), kDenseThreads, 0, st>>>(H, n, k, tau, pw);
-    k_hh_w<<<1, kDenseThreads, 0, st>>>(H, n, k, tau, pw, pw + n);
-    k_hh_rank2<<<dim3((unsigned)((m + 127) / 128), (unsigned)m), 128, 0, st>>>(H, n, k, tau, pw + n);
+  cudaMemsetAsync(hcnt, 0, sizeof(int) * (nb + 1), st);
+  Hh h{H, n, nb, d, e, tau, pw, nullptr, pw + 2 * n, nullptr, nullptr, part, nullptr, hcnt};
+  h.D = pw + 4 * n;
+  h.inv = h.D + nb;
+  h.K = h.inv + 2;
+  h.norms = reinterpret_cast<double*>(h.K + 2);
+  for (int64_t k = 0; k < n; ++k) {
+    k_hh_column<<<(unsigned)((n - k + kTileThreads - 1) / kTileThreads), kTileThreads, 0, st>>>(h, k);
+    if (k + 1 == n) break;
+    const int b0 = (int)((k + 1) / kTile);
+    const int64_t m = nb - b0;
+    k_hh_tile<<<(unsigned)(m * (m + 1) / 2), kTileThreads, 0, st>>>(h, k, b0);
   }
-  k_last_diag<<<1, 1, 0, st>>>(H, n, d);
   // 3. eigenvalues: Gershgorin bounds of T on the host (2n doubles)
   std::vector<double> dh(n), eh(n, 0.0);
   cudaMemcpyAsync(dh.data(), d, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
@@ -490,7 +659,7 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
   gl -= pad;
   gu += pad;
   k_tri_prep<<<grid1(n), 256, 0, st>>>(d, e, (int)n, f32, f32 + n, e2);
-  k_tri_all<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(d, e2, f32, f32 + n, (int)n, gl, gu, tnorm, lam, nfb);
+  k_tri_all<<<(unsigned)((n + 3) / 4), 32, 0, st>>>(d, e2, f32, f32 + n, (int)n, gl, gu, tnorm, lam);
   // 4. eigenvectors
   if (nv > 0) {
     // off-diagonal in the tridiag.cuh convention: eoff[i] couples rows i-1 and i
@@ -501,16 +670,14 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
     k_backtransform<<<(unsigned)nv, kDenseThreads, 0, st>>>(H, n, tau, y, X);
   }
   std::vector<double> out(n);
-  int fallbacks = 0;  // eigenvalues that needed FP64 bisection (multiple or clustered roots)
   cudaMemcpyAsync(out.data(), lam, sizeof(double) * n, cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(&fallbacks, nfb, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (nv > 0) cudaMemcpyAsync(evecs, X, sizeof(double2) * n * nv, cudaMemcpyDeviceToHost, st);
   ce = cudaStreamSynchronize(st);
   if (ce == cudaSuccess) ce = cudaGetLastError();
   cleanup();
   if (ce != cudaSuccess) return cuda_fail(ce, "dense path");
-  // bisection and Newton give the k-th eigenvalue at index k; neighbours
-  // within rounding may come out in either order
+  // the k-th eigenvalue is at index k; neighbours within rounding may come out
+  // in either order
   std::sort(out.begin(), out.end());
   for (int64_t i = 0; i < n; ++i) eigs[i] = out[i];
   *n_out = n;
