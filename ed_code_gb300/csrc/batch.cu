@@ -454,7 +454,7 @@ __global__ void __launch_bounds__(kThreads) k_b_scale(const SegDev* __restrict__
   }
   if (!last_cta(cnt + kCnts * t.seg + kCntAdvance, tb[t.seg + 1] - tb[t.seg])) return;
   __shared__ int ok;
-  __shared__ double d[kMaxSteps + 1], e[kMaxSteps + 1];
+  __shared__ double tsm[(kMaxSteps + 1) * 4];  // TdT of kMaxSteps + 1 rows
   const int jn = j + 1;
   if (threadIdx.x == 0) {
     ok = 1;
@@ -463,18 +463,16 @@ __global__ void __launch_bounds__(kThreads) k_b_scale(const SegDev* __restrict__
   }
   __syncthreads();
   if (jn >= S.m_max || S.tol <= 0 || jn % S.check_every != 0 || jn < 2 * S.want + 2) return;
-  for (int i = threadIdx.x; i < jn; i += blockDim.x) {
-    d[i] = __ldcg(S.alpha + i);
-    e[i] = i > 0 ? __ldcg(S.beta + i) : 0.0;
-  }
+  TdT T(tsm, kMaxSteps + 1);
+  for (int i = threadIdx.x; i < jn; i += blockDim.x) T.set(i, __ldcg(S.alpha + i), i > 0 ? __ldcg(S.beta + i) : 0.0);
   __syncthreads();
   // one warp per wanted eigenvalue (multisection), then its lane 0 runs the
   // inverse iteration
   for (int k = threadIdx.x >> 5; k < S.want; k += blockDim.x >> 5) {
-    const double th = warp_eigenvalue(d, e, jn, k);
+    const double th = warp_eigenvalue(T, 0, jn, k);
     if ((threadIdx.x & 31) == 0) {
       double* y = S.ywork + (int64_t)k * 6 * S.m_max;
-      tridiag_eigenvector(d, e, jn, th, y, y + S.m_max);
+      tridiag_eigenvector(T.d, T.e, jn, th, y, y + S.m_max);
       if (__ldcg(S.beta + jn) * fabs(y[jn - 1]) > S.tol * fmax(1.0, fabs(th))) ok = 0;
     }
   }

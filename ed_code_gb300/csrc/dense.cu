@@ -379,82 +379,13 @@ __global__ void __launch_bounds__(kTileThreads) k_hh_tile(Hh H, int64_t k, int b
 
 // ---- eigenvalues of T: d[0..n-1], off-diagonal e[0..n-2] (row i to i+1) ----
 
-// Counts of eigenvalues below x from the signs of the leading minors
-// p_i = det(T_i - x), p_i = (d_i - x) p_{i-1} - e_{i-1}^2 p_{i-2}: a sign change
-// from p_{i-1} to p_i is an eigenvalue below x (a zero minor counts once
-// whichever sign it is given).  No division, whose FP64 form is a chain of a
-// dozen instructions, and no comparison on the FP64 pipe: the signs and
-// exponents are read as integers, and every four steps the pair is rescaled by a
-// power of two.  A step's chain is one multiply-add.  e2 has no zeros (k_tri_prep).
-__device__ __forceinline__ int count32(const float* __restrict__ d, const float* __restrict__ e2, int n, float x) {
-  float pm = 1.f, p = d[0] - x;
-  int c = (int)(__float_as_uint(p) >> 31);
-  int i = 1;
-  auto step = [&]() {
-    const float pn = fmaf(d[i] - x, p, -(e2[i - 1] * pm));
-    c += (int)((__float_as_uint(pn) ^ __float_as_uint(p)) >> 31);
-    pm = p;
-    p = pn;
-    ++i;
-  };
-  while (i + 4 <= n) {
-    step();
-    step();
-    step();
-    step();
-    const uint32_t ex = max(__float_as_uint(p) & 0x7F800000u, __float_as_uint(pm) & 0x7F800000u);
-    if (ex > (127u + 30u) << 23) {
-      p *= 0x1p-60f;
-      pm *= 0x1p-60f;
-    } else if (ex < (127u - 30u) << 23) {
-      p *= 0x1p60f;
-      pm *= 0x1p60f;
-    }
-  }
-  while (i < n) step();
-  return c;
-}
-
-__device__ __forceinline__ uint32_t exp_of(double x) { return (uint32_t)__double2hiint(x) & 0x7FF00000u; }
-
-__device__ __forceinline__ int count64(const double* __restrict__ d, const double* __restrict__ e2, int n, double x) {
-  double pm = 1.0, p = d[0] - x;
-  int c = (int)((uint32_t)__double2hiint(p) >> 31);
-  int i = 1;
-  auto step = [&]() {
-    const double pn = fma(d[i] - x, p, -(e2[i - 1] * pm));
-    c += (int)((uint32_t)(__double2hiint(pn) ^ __double2hiint(p)) >> 31);
-    pm = p;
-    p = pn;
-    ++i;
-  };
-  while (i + 4 <= n) {
-    step();
-    step();
-    step();
-    step();
-    const uint32_t ex = max(exp_of(p), exp_of(pm));
-    if (ex > (1023u + 300u) << 20) {
-      p *= 0x1p-600;
-      pm *= 0x1p-600;
-    } else if (ex < (1023u - 300u) << 20) {
-      p *= 0x1p600;
-      pm *= 0x1p600;
-    }
-  }
-  while (i < n) step();
-  return c;
-}
-
 __global__ void k_tri_prep(const double* __restrict__ d, const double* __restrict__ e, int n, float* __restrict__ d32,
                            float* __restrict__ e232, double* __restrict__ e2) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     d32[i] = (float)d[i];
     if (i + 1 < n) {
-      // a decoupled row couples by less than any rounding instead (1e-290 and
-      // 1e-30 of |T|^2 ~ 1), so that no minor stays zero
-      e2[i] = fmax(e[i] * e[i], 1e-290);
-      e232[i] = fmaxf((float)e[i] * (float)e[i], 1e-30f);
+      e2[i] = minor_e2(e[i]);
+      e232[i] = minor_e232(e[i]);
     }
   }
 }
@@ -486,8 +417,8 @@ __global__ void __launch_bounds__(32) k_tri_all(const double* __restrict__ d, co
                                                 const float* __restrict__ d32, const float* __restrict__ e232, int n,
                                                 double gl, double gu, double tnorm, double* __restrict__ out) {
   const int k = min(n - 1, (int)((blockIdx.x * 32 + threadIdx.x) >> 3));
-  auto c32 = [&](float x) { return count32(d32, e232, n, x); };
-  auto c64 = [&](double x) { return count64(d, e2, n, x); };
+  auto c32 = [&](float x) { return minor_count(d32, e232, n, x); };
+  auto c64 = [&](double x) { return minor_count(d, e2, n, x); };
   float lo = (float)gl, hi = (float)gu;
   for (int it = 0; it < 16; ++it) {
     const bool run = hi - lo > 4.f * 1.1920929e-7f * fmaxf(fabsf(lo), fabsf(hi));

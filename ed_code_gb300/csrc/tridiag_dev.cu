@@ -7,11 +7,11 @@
 // batch of problems at once (one problem: one T, blockIdx.y):
 //
 //   k_td_values   eigenvalues k of T and of T-hat (T without its first row and
-//                 column), one warp each: multisection on the Sturm count --
-//                 the 32 lanes evaluate the count at 32 interior points of the
-//                 bracket and keep the sub-interval where it passes k, 33x
-//                 narrower per round (Barth, Martin and Wilkinson's bisection,
-//                 Numer. Math. 9 (1967) 386, with the points spread over a warp);
+//                 column), one warp each: multisection on the count of
+//                 eigenvalues below a point -- the 32 lanes evaluate it at 32
+//                 interior points of the bracket and keep the sub-interval where
+//                 it passes k, 33x narrower per round (warp_eigenvalue,
+//                 tridiag.cuh);
 //   k_td_pick     the Ritz values kept: with filtering, Cullum and
 //                 Willoughby's test drops a simple eigenvalue of T that T-hat
 //                 shares (a copy made by lost orthogonality) and keeps one
@@ -20,7 +20,8 @@
 //                 (tridiag.cuh).
 //
 // Every step is deterministic; results do not depend on the other problems in
-// the batch.  All arithmetic is FP64.
+// the batch.  All values are FP64 (FP32 counts only choose where the FP64 ones
+// start).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -39,7 +40,7 @@ int cuda_fail(cudaError_t e, const char* what);
 
 namespace {
 
-constexpr int kTdWarps = 8;
+constexpr int kTdWarps = 2;  // a few: the eigenvalues of one T spread over the SMs' FP64 pipes
 
 // d[i] = Re alpha_i (alpha strided by astride doubles), e[i] = beta_i (e[0] = 0)
 __device__ void load_t(const TdProb& P, double* d, double* e) {
@@ -52,19 +53,16 @@ __device__ void load_t(const TdProb& P, double* d, double* e) {
 __global__ void __launch_bounds__(32 * kTdWarps) k_td_values(const TdProb* __restrict__ probs) {
   const TdProb P = probs[blockIdx.y];
   extern __shared__ double sm[];
-  double* d = sm;
-  double* e = sm + P.m;
   const int idx = blockIdx.x * kTdWarps + (threadIdx.x >> 5);
   if (blockIdx.x * kTdWarps >= P.nc + P.nh) return;  // the whole CTA has no work
-  load_t(P, d, e);
+  TdT T(sm, P.m);
+  for (int i = threadIdx.x; i < P.m; i += blockDim.x)
+    T.set(i, P.alpha[(int64_t)i * P.astride], i > 0 ? P.beta[i] : 0.0);
   __syncthreads();
-  if (idx < P.nc) {
-    const double th = warp_eigenvalue(d, e, P.m, idx);
-    if ((threadIdx.x & 31) == 0) P.vals[idx] = th;
-  } else if (idx < P.nc + P.nh) {
-    const double th = warp_eigenvalue(d + 1, e + 1, P.m - 1, idx - P.nc);
-    if ((threadIdx.x & 31) == 0) P.vals[idx] = th;
-  }
+  if (idx >= P.nc + P.nh) return;
+  const int hat = idx >= P.nc;  // T-hat: rows 1 .. m - 1
+  const double th = warp_eigenvalue(T, hat, P.m, hat ? idx - P.nc : idx);
+  if ((threadIdx.x & 31) == 0) P.vals[idx] = th;
 }
 
 // One warp per problem.  |T| is the largest absolute row sum.  Copies of a
@@ -125,15 +123,15 @@ __global__ void __launch_bounds__(64) k_td_vectors(const TdProb* __restrict__ pr
 cudaError_t td_select_async(const TdProb* probs_dev, int n_probs, int m_max, int nvals_max, TdOut* out_dev,
                             bool vectors, cudaStream_t st) {
   if (n_probs <= 0) return cudaSuccess;
-  const size_t smem = sizeof(double) * 2 * std::max(m_max, 1);
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(k_td_values, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  const size_t smem = sizeof(double) * 2 * std::max(m_max, 1), smem_v = TdT::bytes(std::max(m_max, 1));
+  if (smem_v > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(k_td_values, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_v);
     if (e == cudaSuccess)
       e = cudaFuncSetAttribute(k_td_vectors, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
   const int gx = (std::max(nvals_max, 1) + kTdWarps - 1) / kTdWarps;
-  k_td_values<<<dim3(gx, n_probs), 32 * kTdWarps, smem, st>>>(probs_dev);
+  k_td_values<<<dim3(gx, n_probs), 32 * kTdWarps, smem_v, st>>>(probs_dev);
   k_td_pick<<<n_probs, 32, 0, st>>>(probs_dev, out_dev);
   if (vectors) k_td_vectors<<<n_probs, 64, smem, st>>>(probs_dev, out_dev);
   return cudaGetLastError();
