@@ -19,7 +19,7 @@
 //   k_b_cgs_finish  the segment's <V_k|w> summed over its tiles (FP64); on
 //                   the first pass also whether a second pass is needed (the
 //                   first removed more than 1e-4 of |w|^2)
-//   k_b_cgs_sub     w -= sum_k <V_k|w> V_k; the second pass ends with the
+//   k_b_cgs_sub     w -= sum_k <V_k|w> V_k; the step's last pass ends with the
 //                   tile's |w|^2 for beta_{j+1}
 //   (the three Gram-Schmidt kernels run twice; the second pass returns at
 //   once for a segment that does not need it)
@@ -121,20 +121,26 @@ struct TileDev {
   int64_t row0;
 };
 
+// Sums of a and b over the CTA, in all its threads: one warp each over the
+// threads' values (13 FP64 additions a CTA and sum instead of 24 with a tree of
+// halves; FP64 issue is 16 clocks).
 __device__ __forceinline__ void block_sum2(double& a, double& b) {
-  __shared__ double sa[kThreads], sb[kThreads];
-  sa[threadIdx.x] = a;
-  sb[threadIdx.x] = b;
+  __shared__ double sv[2][kThreads], tot[2];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  sv[0][threadIdx.x] = a;
+  sv[1][threadIdx.x] = b;
   __syncthreads();
-  for (int h = kThreads / 2; h > 0; h >>= 1) {
-    if ((int)threadIdx.x < h) {
-      sa[threadIdx.x] += sa[threadIdx.x + h];
-      sb[threadIdx.x] += sb[threadIdx.x + h];
-    }
-    __syncthreads();
+  if (wid < 2) {
+    double x = 0;
+#pragma unroll
+    for (int q = 0; q < kThreads / 32; ++q) x += sv[wid][32 * q + lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) tot[wid] = x;
   }
-  a = sa[0];
-  b = sb[0];
+  __syncthreads();
+  a = tot[0];
+  b = tot[1];
   __syncthreads();
 }
 
@@ -235,16 +241,29 @@ __global__ void __launch_bounds__(kThreads) k_b_step(const SegDev* __restrict__ 
   const FFScalar a(S.alpha[j]), b(j > 0 ? S.beta[j] : 0.0);
   const float2* v = S.V + (int64_t)j * S.n;
   const float2* vp = j > 0 ? v - S.n : nullptr;
+  float2* __restrict__ w = S.w + t.row0;
+  v += t.row0;
+  if (vp) vp += t.row0;
   FFAcc sr;
-  for (int r = threadIdx.x; r < t.rows; r += blockDim.x) {
-    const int64_t i = t.row0 + r;
-    const float2 y = S.w[i], x = v[i];
-    const float2 p = vp ? vp[i] : make_float2(0.f, 0.f);
+  auto row = [&](int r, float2 y, float2 x, float2 p) {
     const float2 o = make_float2(ff_axpy2(y.x, a, x.x, b, p.x), ff_axpy2(y.y, a, x.y, b, p.y));
-    S.w[i] = o;
+    w[r] = o;
     sr.add_prod(o.x, o.x);
     sr.add_prod(o.y, o.y);
+  };
+  int r = threadIdx.x;
+  for (; r + 3 * kThreads < t.rows; r += 4 * kThreads) {  // four rows in flight
+    float2 y[4], x[4], p[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      y[q] = w[r + q * kThreads];
+      x[q] = v[r + q * kThreads];
+      p[q] = vp ? vp[r + q * kThreads] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) row(r + q * kThreads, y[q], x[q], p[q]);
   }
+  for (; r < t.rows; r += kThreads) row(r, w[r], v[r], vp ? vp[r] : make_float2(0.f, 0.f));
   double s2 = sr.value(), z = 0;
   block_sum2(s2, z);
   if (threadIdx.x == 0) {
@@ -303,7 +322,7 @@ __global__ void __launch_bounds__(kThreads) k_b_cgs_dot(const SegDev* __restrict
   const int K = run ? ss[t.seg].j + 1 : 0, kf = ss[t.seg].kf;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const float2* __restrict__ w = S.w + t.row0;
-  for (int k = kf + blockIdx.y * kWarps + wid; k < K; k += kCgsY * kWarps) {
+  for (int k = kf + blockIdx.y * kWarps + wid; k < K; k += gridDim.y * kWarps) {
     const float2* __restrict__ x = S.V + (int64_t)k * S.n + t.row0;
     KahanAcc sr, si;
     int r = lane;
@@ -343,7 +362,9 @@ __global__ void __launch_bounds__(kThreads) k_b_cgs_dot(const SegDev* __restrict
   }
 }
 
-// CTA (segment, y): q_k = sum of the segment's tile partials, k = y, y + kCgsY, ...
+// CTA (segment, y): q_k = sum of the segment's tile partials, a warp each, k =
+// 8 y + warp, ... (a CTA each took 43 us a step on 160 segments of ten tiles, most
+// of it the trees over 256 threads: 150 steps with a warp each are 8 ms shorter).
 // After the first pass the last of the segment's kCgsY CTAs also decides
 // whether the second pass is needed (Daniel, Gragg, Kaufman and Stewart's
 // test): the first pass removed sum |q_k|^2 from |w|^2; when that is below
@@ -357,14 +378,21 @@ __global__ void __launch_bounds__(kThreads) k_b_cgs_finish(const SegDev* __restr
   if (ss[blockIdx.x].status != kRunning || (pass == 1 && !ss[blockIdx.x].redo)) return;
   const SegDev& S = segs[blockIdx.x];
   const int K = ss[blockIdx.x].j + 1, kf = ss[blockIdx.x].kf;
-  for (int k = kf + blockIdx.y; k < K; k += kCgsY) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int t0 = tb[blockIdx.x], t1 = tb[blockIdx.x + 1];
+  for (int k = kf + blockIdx.y * (kThreads / 32) + wid; k < K; k += kCgsY * (kThreads / 32)) {  // a warp each
     double a = 0, b = 0;
-    for (int t = tb[blockIdx.x] + threadIdx.x; t < tb[blockIdx.x + 1]; t += blockDim.x) {
-      a += part[((int64_t)k * n_tiles + t) * 2];
-      b += part[((int64_t)k * n_tiles + t) * 2 + 1];
+    for (int t = t0 + lane; t < t1; t += 32) {
+      const double2 p = *reinterpret_cast<const double2*>(part + ((int64_t)k * n_tiles + t) * 2);
+      a += p.x;
+      b += p.y;
     }
-    block_sum2(a, b);
-    if (threadIdx.x == 0) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      a += __shfl_down_sync(0xffffffffu, a, o);
+      b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if (lane == 0) {
       S.q[2 * k] = a;
       S.q[2 * k + 1] = b;
     }
@@ -380,9 +408,10 @@ __global__ void __launch_bounds__(kThreads) k_b_cgs_finish(const SegDev* __restr
   }
 }
 
-// w -= sum_k q_k V_k (the first pass; the second only when decided), and
-// after the second, beta_{j+1} = |w| (tile partials of the stored values,
-// closed per segment by the last CTA)
+// w -= sum_k q_k V_k, and in the step's last pass (the first when no second is
+// needed) beta_{j+1} = |w| (tile partials of the stored values, closed per
+// segment by the last CTA).  The second pass returns at once for a segment that
+// does not need it.
 __global__ void __launch_bounds__(kThreads) k_b_cgs_sub(const SegDev* __restrict__ segs,
                                                         const SegState* __restrict__ ss,
                                                         const TileDev* __restrict__ tiles, int pass,
@@ -390,34 +419,30 @@ __global__ void __launch_bounds__(kThreads) k_b_cgs_sub(const SegDev* __restrict
                                                         int* __restrict__ cnt) {
   const TileDev t = tiles[blockIdx.x];
   if (ss[t.seg].status != kRunning) return;
-  const bool sub = pass == 0 || ss[t.seg].redo;
+  const bool redo = ss[t.seg].redo != 0;
+  if (pass == 1 && !redo) return;
   const SegDev& S = segs[t.seg];
   __shared__ float sq[2 * (kMaxSteps + 1)];
   const int K = ss[t.seg].j + 1, kf = ss[t.seg].kf;
-  if (sub) {
-    for (int k = 2 * kf + threadIdx.x; k < 2 * K; k += blockDim.x) sq[k] = (float)S.q[k];
-    __syncthreads();
-  }
+  for (int k = 2 * kf + threadIdx.x; k < 2 * K; k += blockDim.x) sq[k] = (float)S.q[k];
+  __syncthreads();
   // FP32: the q_k are tiny against |w| once the vectors are nearly orthogonal
   FFAcc sr;
   for (int r = threadIdx.x; r < t.rows; r += blockDim.x) {
     const int64_t i = t.row0 + r;
     const float2 y = S.w[i];
     float re = y.x, im = y.y;
-    if (sub) {
-      for (int k = kf; k < K; ++k) {
-        const float2 x = S.V[(int64_t)k * S.n + i];
-        re = fmaf(-sq[2 * k], x.x, fmaf(sq[2 * k + 1], x.y, re));
-        im = fmaf(-sq[2 * k], x.y, fmaf(-sq[2 * k + 1], x.x, im));
-      }
-      S.w[i] = make_float2(re, im);
+#pragma unroll 4
+    for (int k = kf; k < K; ++k) {
+      const float2 x = S.V[(int64_t)k * S.n + i];
+      re = fmaf(-sq[2 * k], x.x, fmaf(sq[2 * k + 1], x.y, re));
+      im = fmaf(-sq[2 * k], x.y, fmaf(-sq[2 * k + 1], x.x, im));
     }
-    if (pass == 1) {
-      sr.add_prod(re, re);
-      sr.add_prod(im, im);
-    }
+    S.w[i] = make_float2(re, im);
+    sr.add_prod(re, re);
+    sr.add_prod(im, im);
   }
-  if (pass == 0) return;
+  if (pass == 0 && redo) return;
   double s2 = sr.value(), z = 0;
   block_sum2(s2, z);
   if (threadIdx.x == 0) {
@@ -1136,7 +1161,8 @@ int rebuild(Batch& B) {
   else k_b_hv<8><<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
   k_b_step<<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, B.d_tb, B.d_part, cnt);
   for (int pass = 0; pass < 2; ++pass) {
-    k_b_cgs_dot<<<dim3(nt, kCgsY), kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, nt, B.d_part, pass);
+    // the second pass is rarely wanted: one CTA a tile then takes all k
+    k_b_cgs_dot<<<dim3(nt, pass == 0 ? kCgsY : 1), kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, nt, B.d_part, pass);
     k_b_cgs_finish<<<dim3(ns, kCgsY), kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tb, nt, B.d_part, pass, cnt);
     k_b_cgs_sub<<<nt, kThreads, 0, B.st>>>(B.d_segs, B.d_state, B.d_tiles, pass, B.d_tb, B.d_part, cnt);
   }

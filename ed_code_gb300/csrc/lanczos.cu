@@ -153,11 +153,23 @@ __global__ void k_sub_multi(T* __restrict__ y, const T* __restrict__ V, int64_t 
   __syncthreads();
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     cd yv = VecTraits<T>::load(y, i);
-    for (int k = 0; k < K; ++k) {
+    int k = 0;
+    for (; k + 8 <= K; k += 8) {  // eight vectors' entries in flight
+      cd vv[8];
+#pragma unroll
+      for (int t = 0; t < 8; ++t) vv[t] = VecTraits<T>::load(V + (int64_t)(k + t) * ld, i);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const double qr = sq[2 * (k + t)], qi = sq[2 * (k + t) + 1];
+        yv.re = fma(-qr, vv[t].re, fma(qi, vv[t].im, yv.re));
+        yv.im = fma(-qr, vv[t].im, fma(-qi, vv[t].re, yv.im));
+      }
+    }
+    for (; k < K; ++k) {
       const cd vv = VecTraits<T>::load(V + (int64_t)k * ld, i);
       const double qr = sq[2 * k], qi = sq[2 * k + 1];
-      yv.re -= qr * vv.re - qi * vv.im;
-      yv.im -= qr * vv.im + qi * vv.re;
+      yv.re = fma(-qr, vv.re, fma(qi, vv.im, yv.re));
+      yv.im = fma(-qr, vv.im, fma(-qi, vv.re, yv.im));
     }
     VecTraits<T>::store(y, i, yv);
   }
