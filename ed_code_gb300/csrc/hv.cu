@@ -175,7 +175,7 @@ size_t free_smem_bytes(const Sector& S, int orb) {
 
 template <typename Real, int kOrb>
 __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const typename CT2<Real>::T* __restrict__ vtab,
-                                                          int n_vals, int table_at,
+                                                          int n_vals, int table_at, int wps,
                                                           const typename CT2<Real>::T* __restrict__ v,
                                                           typename CT2<Real>::T* __restrict__ w) {
   using CT = typename CT2<Real>::T;
@@ -183,6 +183,8 @@ __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const ty
   __shared__ Real nrm[65], nrm_inv[65];
   __shared__ uint32_t q_col[kFreeThreads / 32][kQueue][32];
   __shared__ uint16_t q_id[kFreeThreads / 32][kQueue][32];
+  __shared__ Real part_sum[kFreeThreads / 32][2][32];
+  __shared__ uint64_t part_facs[kFreeThreads / 32][32];
   extern __shared__ __align__(16) uint8_t sm[];
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
     reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
@@ -201,9 +203,11 @@ __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const ty
   auto& qi = q_id[threadIdx.x >> 5];
   const uint64_t pl = l2_evict_last();
   const RowsView<Real> R{nullptr, nullptr, nullptr, tab, v, 0};
-  const int64_t n_p = P.n_p, stride = (int64_t)gridDim.x * blockDim.x;
-  for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < n_p; base += stride) {
-    const int64_t i = base + threadIdx.x;
+  // wps warps share a slice of 32 rows, with every wps-th group each
+  const int64_t n_p = P.n_p;
+  const int wid = threadIdx.x >> 5, part = wid % wps, per_cta = kFreeThreads / 32 / wps;
+  for (int64_t s0 = (int64_t)blockIdx.x * per_cta; s0 * 32 < n_p; s0 += (int64_t)gridDim.x * per_cta) {
+    const int64_t i = (s0 + wid / wps) * 32 + lane;
     const bool live = i < n_p;
     const St s = live ? (St)V.reps[i] : 0;  // no pair is anti-aligned past the end
     CT vi;
@@ -239,7 +243,7 @@ __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const ty
       __syncwarp();
       cnt = 0;
     };
-    for (int g = 0; g < ng; ++g) {
+    for (int g = part; g < ng; g += wps) {
       const PassGroup& gr = H.groups[g];
       const St pm = (St)gr.mask, both = s & pm;
       const bool anti = both != 0 && both != pm;
@@ -271,9 +275,24 @@ __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const ty
       for (int a = 0; a < kAcc / 2; ++a) acc[a][j] += acc[a + kAcc / 2][j];
       sum[j] = kAcc == 2 ? acc[0][j] : acc[0][j] + acc[1 % kAcc][j];
     }
-    if (live) {
+    sum[0] += rest_r;
+    sum[1] += rest_i;
+    if (wps > 1) {
+      part_sum[wid][0][lane] = sum[0];
+      part_sum[wid][1][lane] = sum[1];
+      part_facs[wid][lane] = facs;
+      __syncthreads();
+      if (part == 0)
+        for (int q = 1; q < wps; ++q) {
+          sum[0] += part_sum[wid + q][0][lane];
+          sum[1] += part_sum[wid + q][1][lane];
+          facs += part_facs[wid + q][lane];
+        }
+      __syncthreads();
+    }
+    if (part == 0 && live) {
       const Real f = nrm[li] * nrm_inv[1];
-      w[i] = row_out(sum[0] + rest_r, sum[1] + rest_i, f, (Real)row_ezz(s, facs, P, H), vi);
+      w[i] = row_out(sum[0], sum[1], f, (Real)row_ezz(s, facs, P, H), vi);
     }
   }
 }
@@ -329,9 +348,13 @@ cudaError_t launch_free(const Sector& S, int orb, const void* v, void* w, cudaSt
   const size_t at = align16(pass_smem_bytes(S.P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm));
   const size_t smem = free_smem_bytes<Real>(S, orb);
   auto kern = k_hv_free<Real, kOrb>;
-  const int grid = persistent_grid(kern, smem, S.P.n_p, kFreeThreads);
+  // Up to 1.6e5 rows there are too few warps to hide the chain of searches: 822
+  // rows took 37 us with a warp a slice and take 17 us, 9,250 rows 73 and 28 us,
+  // 112,632 rows 109 and 88 us (FP32).
+  const int wps = S.P.n_p < (int64_t)152 * 32 * 32 ? kFreeThreads / 32 : 1;
+  const int grid = persistent_grid(kern, smem, S.P.n_p * wps, kFreeThreads);
   const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
-  kern<<<grid, kFreeThreads, smem, st>>>(S.V, tab, S.n_vals, (int)at, reinterpret_cast<const CT*>(v),
+  kern<<<grid, kFreeThreads, smem, st>>>(S.V, tab, S.n_vals, (int)at, wps, reinterpret_cast<const CT*>(v),
                                          reinterpret_cast<CT*>(w));
   return cudaGetLastError();
 }
