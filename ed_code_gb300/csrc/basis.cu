@@ -101,7 +101,8 @@ __global__ void __launch_bounds__(kBuildThreads) k_basis_count(SectorView V, uin
 
 template <bool kTorus>
 __global__ void __launch_bounds__(kBuildThreads) k_basis_emit(SectorView V, const uint32_t* __restrict__ counts,
-                                                              uint64_t* __restrict__ reps, uint8_t* __restrict__ lid) {
+                                                              uint64_t* __restrict__ reps, uint8_t* __restrict__ lid,
+                                                              unsigned long long* __restrict__ lids) {
   __shared__ SectorParams P;
   extern __shared__ __align__(16) uint8_t sm[];
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
@@ -111,6 +112,7 @@ __global__ void __launch_bounds__(kBuildThreads) k_basis_emit(SectorView V, cons
   const int64_t n_recs = P.n_recs;
   for (int64_t r = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n_recs; r += (int64_t)gridDim.x * blockDim.x) {
     if (counts[r] == 0) continue;
+    unsigned long long seen = 0;
     const RankRec rec = V.recs[r];
     const int64_t lin0 = r * kRecBits;
     const int64_t rem = P.n_configs - lin0;
@@ -120,11 +122,14 @@ __global__ void __launch_bounds__(kBuildThreads) k_basis_emit(SectorView V, cons
     for (int idx = 0; idx < n; ++idx) {
       if ((rec.bits[idx >> 5] >> (idx & 31)) & 1u) {
         reps[q] = t;
-        lid[q] = (uint8_t)allowed<kTorus>(t, P, T, V.n_chunks);
+        const int l = allowed<kTorus>(t, P, T, V.n_chunks);
+        lid[q] = (uint8_t)l;
+        seen |= 1ull << (l - 1);
         ++q;
       }
       if (idx + 1 < n) t = next_same_popcount(t);
     }
+    if (seen & ~__ldcg(lids)) atomicOr(lids, seen);  // rarely new
   }
 }
 
@@ -271,7 +276,8 @@ cudaError_t build_basis(Sector& S, std::string& err) {
   const int64_t n_chunks = (n_recs + kScanChunk - 1) / kScanChunk;
   cudaError_t e = cudaMalloc(&counts, sizeof(uint32_t) * std::max<int64_t>(1, n_recs));
   if (e == cudaSuccess) e = cudaMalloc(&chunk, sizeof(uint32_t) * std::max<int64_t>(1, n_chunks));
-  if (e == cudaSuccess) e = cudaMalloc(&total, sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&total, 2 * sizeof(unsigned long long));  // a total, the stabiliser counts
+  if (e == cudaSuccess) e = cudaMemsetAsync(total, 0, 2 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) {
     err = "basis build: scratch allocation failed";
     cudaFree(counts); cudaFree(chunk); cudaFree(total);
@@ -309,14 +315,17 @@ cudaError_t build_basis(Sector& S, std::string& err) {
     if (torus) {
       cudaFuncSetAttribute(k_basis_emit<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       k_basis_emit<true><<<grid_for((const void*)k_basis_emit<true>, smem, n_recs), kBuildThreads, smem, st>>>(
-          S.V, counts, S.reps, S.lid);
+          S.V, counts, S.reps, S.lid, total + 1);
     } else {
       cudaFuncSetAttribute(k_basis_emit<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       k_basis_emit<false><<<grid_for((const void*)k_basis_emit<false>, smem, n_recs), kBuildThreads, smem, st>>>(
-          S.V, counts, S.reps, S.lid);
+          S.V, counts, S.reps, S.lid, total + 1);
     }
   }
-  e = cudaStreamSynchronize(st);
+  unsigned long long lids = 0;
+  e = cudaMemcpyAsync(&lids, total + 1, sizeof(lids), cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  S.lids = lids;
   // The Lin-indexed records are not needed past this point.
   cudaFree(S.recs);
   S.device_bytes -= sizeof(RankRec) * std::max<int64_t>(1, n_recs);

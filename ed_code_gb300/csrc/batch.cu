@@ -93,7 +93,7 @@ struct SegDev {
   const double* nrm_inv;
   float2* V;              // (m_max + 1) x n
   float2* w;
-  float2* u;
+  float2* u;              // V_j / norm (nullptr: folded rows gather V_j itself)
   double* alpha;          // m_max + 1
   double* beta;           // m_max + 2
   double* q;              // 2 (m_max + 1): reorthogonalisation coefficients
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kThreads) k_b_hv(const SegDev* __restrict__ se
   const SegDev& S = segs[t.seg];
   const float2* v = S.V + (int64_t)ss[t.seg].j * S.n;
   const uint64_t pl = l2_evict_last();
-  const RowsView<float> R{S.row_ptr, S.col, S.vid, S.vtab, S.u, S.pack_cb};
+  const RowsView<float> R{S.row_ptr, S.col, S.vid, S.vtab, S.u ? S.u : v, S.pack_cb};
   FFAcc sr, si;
   for (int r0 = 0; r0 < t.rows; r0 += kThreads) {  // the tile starts at a multiple of 32
     const int r = r0 + threadIdx.x;
@@ -474,8 +474,10 @@ __global__ void __launch_bounds__(kThreads) k_b_scale(const SegDev* __restrict__
     const float2 y = S.w[i];
     const float2 x = make_float2(fmaf(y.x, s.l, __fmul_rn(y.x, s.h)), fmaf(y.y, s.l, __fmul_rn(y.y, s.h)));
     vn[i] = x;
-    const float ni = (float)S.nrm_inv[S.lid[i]];
-    S.u[i] = make_float2(x.x * ni, x.y * ni);
+    if (S.u) {
+      const float ni = (float)S.nrm_inv[S.lid[i]];
+      S.u[i] = make_float2(x.x * ni, x.y * ni);
+    }
   }
   if (!last_cta(cnt + kCnts * t.seg + kCntAdvance, tb[t.seg + 1] - tb[t.seg])) return;
   __shared__ int ok;
@@ -537,8 +539,10 @@ __global__ void __launch_bounds__(kThreads) k_b_start(float2* __restrict__ V0, c
     const float2 v = make_float2(fmaf(x[i].x, inv.l, __fmul_rn(x[i].x, inv.h)),
                                  fmaf(x[i].y, inv.l, __fmul_rn(x[i].y, inv.h)));
     V0[i] = v;
-    const float ni = (float)nrm_inv[lid[i]];
-    u[i] = make_float2(v.x * ni, v.y * ni);
+    if (u) {
+      const float ni = (float)nrm_inv[lid[i]];
+      u[i] = make_float2(v.x * ni, v.y * ni);
+    }
   }
 }
 
@@ -561,7 +565,7 @@ struct FinVec {
   const double* nrm;
   const double* nrm_inv;
   const double2* x;
-  double2* u;
+  double2* u;           // x / norm (nullptr: folded rows gather x itself)
   double2* hx;
   double* res;  // |x|^2, <x|Hx>, theta, residual
   int64_t n;
@@ -625,6 +629,7 @@ constexpr int64_t kFinCap = 1 << 23;  // vector entries per group of finishing s
 __global__ void __launch_bounds__(kThreads) k_f_u(const FinVec* __restrict__ vs, const FinTile* __restrict__ ts) {
   const FinTile t = ts[blockIdx.x];
   const FinVec& V = vs[t.v];
+  if (!V.u) return;
   for (int r = threadIdx.x; r < t.rows; r += blockDim.x) {
     const int64_t i = t.row0 + r;
     const double s = V.nrm_inv[V.lid[i]];
@@ -638,7 +643,7 @@ __global__ void __launch_bounds__(kThreads) k_f_hv(const FinVec* __restrict__ vs
   const FinTile t = ts[blockIdx.x];
   const FinVec& V = vs[t.v];
   const uint64_t pl = l2_evict_last();
-  const RowsView<double> R{V.row_ptr, V.col, V.vid, V.vtab, V.u, V.pack_cb};
+  const RowsView<double> R{V.row_ptr, V.col, V.vid, V.vtab, V.u ? V.u : V.x, V.pack_cb};
   Acc s0, s1;
   for (int r0 = 0; r0 < t.rows; r0 += kThreads) {  // tiles start at multiples of 32 rows
     const int r = r0 + threadIdx.x;
@@ -994,7 +999,7 @@ void finish_stopped(Batch& B) {
     Segment& g = B.segs[idx[i]];
     const int m = g.st.j, na = sel[i].na;
     const Sector& S = g.sec->s;
-    if (g.d.n <= kFinMaxN && S.vtab64) {
+    if (g.d.n <= kFinMaxN && S.rtab64) {
       const int64_t need = g.d.n * na;
       if (fel + need > kFinCap) flush();
       if (!B.fx) {
@@ -1026,13 +1031,13 @@ void finish_stopped(Batch& B) {
         v.row_ptr = S.row_ptr;
         v.col = S.col;
         v.vid = S.vid;
-        v.vtab = reinterpret_cast<const double2*>(S.vtab64);
+        v.vtab = S.rtab64;
         v.ezz = S.ezz;
         v.lid = S.lid;
         v.nrm = g.d.nrm;
         v.nrm_inv = g.d.nrm_inv;
         v.x = B.fx + fel + (int64_t)q * g.d.n;
-        v.u = B.fu + fel + (int64_t)q * g.d.n;
+        v.u = S.folded ? nullptr : B.fu + fel + (int64_t)q * g.d.n;
         v.hx = B.fhx + fel + (int64_t)q * g.d.n;
         v.res = B.fin.res + 4 * (off[i] + q);
         v.n = g.d.n;
@@ -1254,7 +1259,7 @@ int edg_batch_add(edg_batch* bh, edg_sector* sec, const edg_batch_request* req) 
   d.col = S.col;
   d.vid = S.vid;
   d.pack_cb = S.pack_cb;
-  d.vtab = S.vtab32;
+  d.vtab = S.rtab32;
   d.ezz = S.ezz;
   d.lid = S.lid;
   d.nrm = reinterpret_cast<const double*>(reinterpret_cast<const char*>(S.dP) + offsetof(SectorParams, nrm));
@@ -1266,7 +1271,7 @@ int edg_batch_add(edg_batch* bh, edg_sector* sec, const edg_batch_request* req) 
   d.tol = req->tol;
   cudaError_t e = cudaMalloc(&d.V, sizeof(float2) * n * (m + 1));
   if (e == cudaSuccess) e = cudaMalloc(&d.w, sizeof(float2) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&d.u, sizeof(float2) * n);
+  if (e == cudaSuccess && !S.folded) e = cudaMalloc(&d.u, sizeof(float2) * n);
   if (e == cudaSuccess) e = cudaMalloc(&d.alpha, sizeof(double) * (m + 1));
   if (e == cudaSuccess) e = cudaMalloc(&d.beta, sizeof(double) * (m + 2));
   if (e == cudaSuccess) e = cudaMalloc(&d.q, sizeof(double) * 2 * (m + 1));

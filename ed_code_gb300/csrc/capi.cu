@@ -126,6 +126,7 @@ static int create_sector(const edg_model* m, int n_ones, int kx, int ky, int kz,
   P.n_configs = (int64_t)binomial(N, n_ones);
   P.n_recs = (P.n_configs + kRecBits - 1) / kRecBits;
   P.ChCh = m->ChCh;
+  P.n_stab = 1;
 
   // Row-major torus test: T1 = +x, T2 = +y with Lx = L1, Ly = L2 (2-D only).
   {
@@ -377,6 +378,7 @@ static int create_sector(const edg_model* m, int n_ones, int kx, int ky, int kz,
     S.V.order = reinterpret_cast<const uint16_t*>(dev + oo);
     S.V.remap = reinterpret_cast<const uint16_t*>(dev + orm);
     S.n_vals = (int)T.v64.size();
+    S.values_host = T.v64;
   } else {
     S.values_err = T.why;
   }
@@ -484,7 +486,7 @@ int edg_sector_get_info(const edg_sector* s, edg_sector_info* info) {
   info->ctas_per_sm = s->s.col ? s->s.csr_cps : 0;
   info->pipelined = s->s.col ? s->s.csr_pipe : 0;
   info->entry_bytes = s->s.col ? (s->s.pack_cb ? 4 : 6) : 0;
-  info->n_values = s->s.col ? s->s.n_vals : 0;
+  info->n_values = s->s.col ? s->s.n_rvals : 0;
   return EDG_OK;
 }
 
@@ -606,6 +608,7 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
            reinterpret_cast<uintptr_t>(va.devicePointer) % (fp64 ? 16 : 8) == 0)
     v_dev = va.devicePointer;
   const bool u_done = S.col && v_dev;
+  const void* u = S.folded ? S.host_in.ptr : S.ubuf.ptr;
   e = u_done ? launch_u_in(S, v_dev, S.host_in.ptr, fp64, S.stream)
              : cudaMemcpyAsync(S.host_in.ptr, v, bytes, cudaMemcpyHostToDevice, S.stream);
   // w in page-locked host memory that the device can address (cudaHostAlloc,
@@ -618,7 +621,7 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
   else if (wa.type == cudaMemoryTypeHost)
     w_dev = wa.devicePointer;
   if (e == cudaSuccess && w_dev) {
-    e = u_done ? launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, w_dev, fp64, 0, n, S.stream)
+    e = u_done ? launch_hv_rows(S, S.host_in.ptr, u, w_dev, fp64, 0, n, S.stream)
                : launch_hv(S, S.host_in.ptr, w_dev, fp64, S.stream);
   } else if (S.col && n >= (1 << 20)) {
     // rows in row order: the w rows of chunk c go back to the host while the
@@ -627,11 +630,11 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
     for (int c = 0; c < kChunks && e == cudaSuccess; ++c)
       if (!S.chunk_done[c]) e = cudaEventCreateWithFlags(&S.chunk_done[c], cudaEventDisableTiming);
     const size_t elem = fp64 ? 16 : 8;
-    if (e == cudaSuccess && !u_done) e = launch_u(S, S.host_in.ptr, S.ubuf.ptr, fp64, S.stream);
+    if (e == cudaSuccess && !u_done && !S.folded) e = launch_u(S, S.host_in.ptr, S.ubuf.ptr, fp64, S.stream);
     for (int c = 0; c < kChunks && e == cudaSuccess; ++c) {
       // whole slices of 32 rows
       const int64_t r0 = n * c / kChunks / 32 * 32, r1 = c + 1 == kChunks ? n : n * (c + 1) / kChunks / 32 * 32;
-      e = launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, S.host_out.ptr, fp64, r0, r1, S.stream);
+      e = launch_hv_rows(S, S.host_in.ptr, u, S.host_out.ptr, fp64, r0, r1, S.stream);
       if (e == cudaSuccess) e = cudaEventRecord(S.chunk_done[c], S.stream);
       if (e == cudaSuccess) e = cudaStreamWaitEvent(S.copy_stream, S.chunk_done[c], 0);
       if (e == cudaSuccess)
@@ -641,7 +644,7 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(S.copy_stream);
   } else {
     if (e == cudaSuccess)
-      e = u_done ? launch_hv_rows(S, S.host_in.ptr, S.ubuf.ptr, S.host_out.ptr, fp64, 0, n, S.stream)
+      e = u_done ? launch_hv_rows(S, S.host_in.ptr, u, S.host_out.ptr, fp64, 0, n, S.stream)
                  : launch_hv(S, S.host_in.ptr, S.host_out.ptr, fp64, S.stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(w, S.host_out.ptr, bytes, cudaMemcpyDeviceToHost, S.stream);
   }

@@ -71,7 +71,7 @@ __global__ void k_dense_rows(const uint64_t* __restrict__ row_ptr, const uint32_
         const uint32_t e = col[t];
         const uint32_t j = vid ? e : e & ((1u << cb) - 1u);
         const double2 c = vtab[vid ? (uint32_t)vid[t] : e >> cb];
-        const double sc = ni * nrm_inv[lid[j]];
+        const double sc = nrm_inv ? ni * nrm_inv[lid[j]] : ni;  // nullptr: in the values
         double2* h = H + (int64_t)j * n + i;
         h->x += c.x * sc;
         h->y += c.y * sc;
@@ -541,7 +541,8 @@ int solve_dense_device(Sector& S, double* eigs, int64_t cap, int64_t* n_out, dou
                                                         offsetof(SectorParams, nrm));
     const double* nrm_inv = reinterpret_cast<const double*>(reinterpret_cast<const char*>(S.dP) +
                                                             offsetof(SectorParams, nrm_inv));
-    k_dense_rows<<<grid1(n), 256, 0, st>>>(S.row_ptr, S.col, S.vid, S.pack_cb, S.vtab64, S.ezz, S.lid, nrm, nrm_inv,
+    k_dense_rows<<<grid1(n), 256, 0, st>>>(S.row_ptr, S.col, S.vid, S.pack_cb, S.rtab64, S.ezz, S.lid, nrm,
+                                           S.folded ? nullptr : nrm_inv,
                                            n, H);
   } else {
     for (int64_t j = 0; j < n && ce == cudaSuccess; ++j) {

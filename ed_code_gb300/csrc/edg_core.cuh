@@ -126,8 +126,12 @@ struct SectorParams {
   int64_t n_targets;
   // Distinct values of TermGroup::fac (one per coupling strength); n_facs >
   // kMaxFacs: facs is not filled and rows sum fac itself.
-  int n_facs, pad3;
+  int n_facs;
+  // Stored rows whose values include 1/norm of the target (targets.cu): the
+  // number of distinct stabiliser counts and the index of each; else 1 and 0.
+  int n_stab;
   double facs[kMaxFacs];
+  uint8_t stab_idx[72];
 };
 
 // --------------------------------------------------------------------------

@@ -79,6 +79,7 @@ struct Sector {
   void* values = nullptr;       // value tables (value_tables), one allocation
   double2* vtab64 = nullptr;    // in it: the distinct pair coefficient x phase values
   float2* vtab32 = nullptr;
+  std::vector<double2> values_host;
   int n_vals = 0;               // 0: the tables do not cover the Hamiltonian (values_err)
   std::string values_err;
   size_t device_bytes = 0;
@@ -100,7 +101,13 @@ struct Sector {
   uint16_t* vid = nullptr;      // value ids; null when the entries are packed
   int pack_cb = 0;              // column bits of a packed entry (0: split arrays)
   double* ezz = nullptr;        // diagonal of each row
-  DeviceBuffer ubuf;            // u = v / norm scratch
+  uint64_t lids = 0;            // the stabiliser counts that occur: bit lid - 1
+  void* row_values = nullptr;   // folded rows' value table
+  double2* rtab64 = nullptr;    // the values the rows' ids refer to: vtab64/32, or with folded
+  float2* rtab32 = nullptr;     // their products with 1/norm of each stabiliser count
+  int n_rvals = 0;
+  bool folded = false;          // rows gather v itself, no u
+  DeviceBuffer ubuf;            // u = v / norm scratch (not folded)
   DeviceBuffer ublk;            // the same for edg_hv_block's interleaved vectors
   size_t targets_bytes = 0;
   int csr_lpr = 8;              // 8, 16 or 32: csr_lpr / 2 entries of a row in flight: edg_sector_tune
@@ -166,13 +173,13 @@ void free_targets(Sector& S);
 cudaError_t launch_hv_stored(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st);
 // hv_block.cu: W = H V for nv = 2 or 4 vectors interleaved by row, u the n_p x nv scratch
 cudaError_t launch_hv_block(const Sector& S, const void* v, void* w, int nv, bool fp64, void* u, cudaStream_t st);
-// stored rows: u = v / norm, and rows [r0, r1) of w = H v from v and u (r0 a
-// multiple of 32)
+// stored rows: u = v / norm (not folded), and rows [r0, r1) of w = H v from v and
+// u, or v again when folded (r0 a multiple of 32)
 cudaError_t launch_u(const Sector& S, const void* v, void* u, bool fp64, cudaStream_t st);
 cudaError_t launch_hv_rows(const Sector& S, const void* v, const void* u, void* w, bool fp64, int64_t r0, int64_t r1,
                            cudaStream_t st);
-// stored rows: u = v / norm and v_dst = v from a v_src the device reads in
-// place (mapped page-locked host memory)
+// stored rows: v_dst = v from a v_src the device reads in place (mapped
+// page-locked host memory), and u = v / norm unless folded
 cudaError_t launch_u_in(const Sector& S, const void* v_src, void* v_dst, bool fp64, cudaStream_t st);
 int tune_rows(Sector& S, int lpr, int* chosen, double* ms_out);
 int hv_grid_blocks(bool fp64, bool torus, bool chch);

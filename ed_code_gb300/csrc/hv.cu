@@ -28,6 +28,7 @@
 
 #include "csr_row.cuh"
 #include "hv_common.cuh"
+#include "launch.cuh"
 #include "row_walk.cuh"
 
 namespace edg {
@@ -321,14 +322,14 @@ __global__ void __launch_bounds__(kHvThreads) k_count_offdiag(SectorView V, unsi
 }
 
 template <typename K>
-int persistent_grid(K kernel, size_t smem, int64_t rows, int threads = kHvThreads) {
+int persistent_grid(K kernel, size_t smem, int64_t rows) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kHvThreads, smem);
   if (per_sm < 1) per_sm = 1;
-  int64_t want = (rows + threads - 1) / threads;
+  int64_t want = (rows + kHvThreads - 1) / kHvThreads;
   return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
 }
 
@@ -352,7 +353,11 @@ cudaError_t launch_free(const Sector& S, int orb, const void* v, void* w, cudaSt
   // rows took 37 us with a warp a slice and take 17 us, 9,250 rows 73 and 28 us,
   // 112,632 rows 109 and 88 us (FP32).
   const int wps = S.P.n_p < (int64_t)152 * 32 * 32 ? kFreeThreads / 32 : 1;
-  const int grid = persistent_grid(kern, smem, S.P.n_p * wps, kFreeThreads);
+  // shared memory: at most the walk's tables (48 KB of permutations), 256 groups,
+  // 1,024 chirality sites and 2,048 values
+  const Resident r = resident((const void*)kern, kFreeThreads, smem, 128 * 1024);
+  const int64_t want = (S.P.n_p * wps + kFreeThreads - 1) / kFreeThreads;
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)r.sms * r.per_sm));
   const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
   kern<<<grid, kFreeThreads, smem, st>>>(S.V, tab, S.n_vals, (int)at, wps, reinterpret_cast<const CT*>(v),
                                          reinterpret_cast<CT*>(w));

@@ -55,10 +55,19 @@ template <typename Real, int NV, int kPol, int kFmt>
 cudaError_t launch_blk(const Sector& S, const void* v, void* w, void* u, cudaStream_t st) {
   using CT = typename CT2<Real>::T;
   const int64_t n = S.P.n_p;
+  constexpr int kG = sizeof(Real) == 8 && NV == 4 ? 2 : 4;
+  // rows that gather v itself: by 16-byte loads, so from a copy of an FP32 v that
+  // starts between two of them
+  if (S.folded) {
+    if (u) {
+      const cudaError_t e = cudaMemcpyAsync(u, v, sizeof(CT) * n * NV, cudaMemcpyDeviceToDevice, st);
+      if (e != cudaSuccess) return e;
+    }
+    return launch_rows_k<Real, NV, true, kPol, kFmt, 4, kG, true>(S, v, u ? u : v, w, 0, n, st);
+  }
   k_u_scale_blk<Real, NV><<<(int)std::min<int64_t>((n * NV + 255) / 256, 152 * 32), 256, 0, st>>>(
       reinterpret_cast<const CT*>(v), S.lid, params_field(S, offsetof(SectorParams, nrm_inv)), n,
       reinterpret_cast<CT*>(u));
-  constexpr int kG = sizeof(Real) == 8 && NV == 4 ? 2 : 4;
   return launch_rows_k<Real, NV, true, kPol, kFmt, 4, kG, true>(S, v, u, w, 0, n, st);
 }
 
@@ -74,7 +83,7 @@ cudaError_t launch_blk2(const Sector& S, const void* v, void* w, void* u, cudaSt
 }  // namespace
 
 // W = H V for nv = 2 or 4 interleaved vectors on the stored rows; u is the
-// caller's n_p * nv scratch.  The value table must fit in shared memory.
+// caller's n_p * nv scratch (nullptr: folded rows and an aligned v need none).  The value table must fit in shared memory.
 cudaError_t launch_hv_block(const Sector& S, const void* v, void* w, int nv, bool fp64, void* u, cudaStream_t st) {
   if (fp64) return nv == 2 ? launch_blk2<double, 2>(S, v, w, u, st) : launch_blk2<double, 4>(S, v, w, u, st);
   return nv == 2 ? launch_blk2<float, 2>(S, v, w, u, st) : launch_blk2<float, 4>(S, v, w, u, st);
@@ -91,10 +100,11 @@ extern "C" int edg_hv_block(edg_sector* s, const void* v, void* w, int n_vectors
   Sector& S = s->s;
   if (!S.col) return fail(EDG_ERR_INVALID, "edg_hv_block needs stored rows (edg_sector_build_targets)");
   const bool fp64 = dtype == EDG_C128;
-  if ((size_t)S.n_vals * (fp64 ? 16 : 8) > 96 * 1024)
+  if ((size_t)S.n_rvals * (fp64 ? 16 : 8) > 96 * 1024)
     return fail(EDG_ERR_UNSUPPORTED, "edg_hv_block: value table larger than 96 KB");
   const size_t bytes = (size_t)S.P.n_p * n_vectors * (fp64 ? 16 : 8);
-  if (S.ublk.bytes < bytes) {
+  const bool scratch = !S.folded || reinterpret_cast<uintptr_t>(v) % 16 != 0;
+  if (scratch && S.ublk.bytes < bytes) {
     if (S.ublk.ptr) cudaFree(S.ublk.ptr);
     S.ublk = DeviceBuffer{};
     if (cudaMalloc(&S.ublk.ptr, bytes) != cudaSuccess) {
@@ -104,7 +114,7 @@ extern "C" int edg_hv_block(edg_sector* s, const void* v, void* w, int n_vectors
     S.ublk.bytes = bytes;
     S.device_bytes += bytes;
   }
-  const cudaError_t e = launch_hv_block(S, v, w, n_vectors, fp64, S.ublk.ptr, (cudaStream_t)stream);
+  const cudaError_t e = launch_hv_block(S, v, w, n_vectors, fp64, scratch ? S.ublk.ptr : nullptr, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "edg_hv_block launch");
   return EDG_OK;
 }

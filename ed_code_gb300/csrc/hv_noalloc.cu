@@ -94,7 +94,8 @@ extern "C" int edg_hv_noalloc(edg_sector* s, const void* v, void* w, int dtype, 
   e = scratch_address(dev, &u);
   if (e != cudaSuccess) return cuda_fail(e, "edg_hv_noalloc: cudaGetSymbolAddress of the scratch array");
   const cudaStream_t st = (cudaStream_t)stream;
-  e = launch_u(S, v, u, dtype == EDG_C128, st);
+  if (S.folded) u = const_cast<void*>(v);  // the rows gather v itself
+  else e = launch_u(S, v, u, dtype == EDG_C128, st);
   if (e == cudaSuccess) e = launch_hv_rows(S, v, u, w, dtype == EDG_C128, 0, S.P.n_p, st);
   if (e != cudaSuccess) return cuda_fail(e, "edg_hv_noalloc launch");
   return EDG_OK;

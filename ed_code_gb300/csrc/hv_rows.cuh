@@ -7,6 +7,7 @@
 
 #include "csr_row.cuh"
 #include "edg_sector.cuh"
+#include "launch.cuh"
 
 namespace edg {
 
@@ -14,7 +15,8 @@ namespace {
 
 constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
 
-// w_i = norm_i * sum_t vtab[vid_t] * u[col_t] + Ezz_i * v_i for the rows
+// w_i = norm_i * sum_t vtab[vid_t] * u[col_t] + Ezz_i * v_i (u = v / norm, or v
+// itself where the values include the targets' 1/norm) for the rows
 // [row0, row1) of n, row0 a multiple of 32: a warp per slice of 32 rows, or
 // wps warps with a share of its slots each (warps_per_slice).  NV vectors are
 // interleaved by row (entry i of vector q at i * NV + q); each gets the bits
@@ -97,7 +99,7 @@ inline const double* params_field(const Sector& S, size_t offset) {
 template <typename Real>
 RowsView<Real> rows_of(const Sector& S, const void* u) {
   using CT = typename CT2<Real>::T;
-  const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
+  const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.rtab64 : (const void*)S.rtab32);
   return RowsView<Real>{S.row_ptr, S.col, S.vid, tab, reinterpret_cast<const CT*>(u), S.pack_cb};
 }
 
@@ -105,15 +107,10 @@ RowsView<Real> rows_of(const Sector& S, const void* u) {
 // per SM when cap > 0, no more than the slices need.
 template <typename K>
 int rows_grid(K kernel, size_t smem, int64_t slices, int per_cta, int cap) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kRowThreads, smem);
-  if (cap > 0 && per_sm > cap) per_sm = cap;
-  if (per_sm < 1) per_sm = 1;
+  Resident r = resident((const void*)kernel, kRowThreads, smem, 96 * 1024);
+  if (cap > 0 && r.per_sm > cap) r.per_sm = cap;
   const int64_t want = (slices + per_cta - 1) / per_cta;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)r.sms * r.per_sm));
 }
 
 // rows [r0, r1) of w = H v from u = v / norm
@@ -123,10 +120,10 @@ cudaError_t launch_rows_k(const Sector& S, const void* v, const void* u, void* w
   using CT = typename CT2<Real>::T;
   if (r1 <= r0) return cudaGetLastError();
   const int wps = warps_per_slice(S.P.n_p);
-  const size_t smem = kSmemTab ? sizeof(CT) * S.n_vals : 0;
+  const size_t smem = kSmemTab ? sizeof(CT) * S.n_rvals : 0;
   auto kern = k_hv_rows<Real, NV, kSmemTab, kPol, kFmt, kU, kG, kPipe>;
   const int grid = rows_grid(kern, smem, (r1 - r0 + 31) / 32, kRowWarps / wps, S.csr_cps);
-  kern<<<grid, kRowThreads, smem, st>>>(rows_of<Real>(S, u), S.n_vals, S.ezz, S.lid,
+  kern<<<grid, kRowThreads, smem, st>>>(rows_of<Real>(S, u), S.n_rvals, S.ezz, S.lid,
                                         params_field(S, offsetof(SectorParams, nrm)), r0, r1, wps,
                                         reinterpret_cast<const CT*>(v), reinterpret_cast<CT*>(w));
   return cudaGetLastError();

@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb,
       }
       const int64_t j = position(o, V, P);
       if (j < 0) continue;
-      const uint32_t id = value_id(s, gr, o.g, V, P, H);
+      const uint32_t id = value_id(s, gr, o.g, V, P, H) * P.n_stab + P.stab_idx[o.stab];
       const uint2 sk = slot[cnt++];
       const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
       if (cb) {
@@ -230,6 +230,7 @@ __global__ void k_u_scale(const typename CT2<Real>::T* __restrict__ v, const uin
 // diagonal term: one pass over the host link, four loads in flight per
 // thread, instead of a copy-engine copy followed by the u pass.  u gets the
 // bits k_u_scale gives it.
+// u may be nullptr (rows that gather v itself).
 template <typename Real>
 __global__ void k_u_scale_in(const typename CT2<Real>::T* __restrict__ v, const uint8_t* __restrict__ lid,
                              const double* __restrict__ nrm_inv_tab, int64_t n, typename CT2<Real>::T* __restrict__ vd,
@@ -248,6 +249,7 @@ __global__ void k_u_scale_in(const typename CT2<Real>::T* __restrict__ v, const 
     for (int k = 0; k < 4; ++k) {
       const int64_t r = i + k * stride;
       vd[r] = x[k];
+      if (!u) continue;
       const Real s = tab[lid[r]];
       x[k].x *= s;
       x[k].y *= s;
@@ -257,6 +259,7 @@ __global__ void k_u_scale_in(const typename CT2<Real>::T* __restrict__ v, const 
   for (; i < n; i += stride) {
     CT x = v[i];
     vd[i] = x;
+    if (!u) continue;
     const Real s = tab[lid[i]];
     x.x *= s;
     x.y *= s;
@@ -287,7 +290,7 @@ template <typename Real, int kPol, int kFmt>
 cudaError_t launch_rows_f(const Sector& S, const void* v, const void* u, void* w, int64_t r0, int64_t r1,
                           cudaStream_t st) {
   constexpr int kMost = sizeof(Real) == 4 ? 16 : 8;
-  if (sizeof(typename CT2<Real>::T) * S.n_vals > 96 * 1024)
+  if (sizeof(typename CT2<Real>::T) * S.n_rvals > 96 * 1024)
     return launch_rows_k<Real, 1, false, kPol, kFmt, 8, 8, false>(S, v, u, w, r0, r1, st);
   if (S.csr_pipe) switch (S.csr_lpr) {
       case 8: return launch_rows_k<Real, 1, true, kPol, kFmt, 4, 4, true>(S, v, u, w, r0, r1, st);
@@ -323,7 +326,7 @@ int64_t gcd64(int64_t a, int64_t b) {
 }  // namespace
 
 void free_targets(Sector& S) {
-  void* ptrs[] = {S.row_ptr, S.col, S.vid, S.ezz, S.ubuf.ptr};
+  void* ptrs[] = {S.row_ptr, S.col, S.vid, S.ezz, S.row_values, S.ubuf.ptr};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   S.row_ptr = nullptr;
@@ -331,6 +334,11 @@ void free_targets(Sector& S) {
   S.vid = nullptr;
   S.pack_cb = 0;
   S.ezz = nullptr;
+  S.row_values = nullptr;
+  S.rtab64 = nullptr;
+  S.rtab32 = nullptr;
+  S.n_rvals = 0;
+  S.folded = false;
   S.ubuf = DeviceBuffer{};
   S.P.n_targets = 0;
   S.device_bytes -= S.targets_bytes;
@@ -456,20 +464,65 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   // Packed entries when the value ids and the columns fit one u32 together:
   // vb bits of value id above cb = 32 - vb column bits, n_p < 2^cb.
   // EDG_ROW_FORMAT=split keeps the two arrays (for comparisons).
-  int vb = 1;
-  while ((1 << vb) < S.n_vals) ++vb;
+  auto pack_bits = [&](int64_t values) {
+    int vb = 1;
+    while (((int64_t)1 << vb) < values) ++vb;
+    return vb < 32 && P.n_p < (int64_t(1) << (32 - vb)) ? 32 - vb : 0;
+  };
+  // Folded rows: the values include the target's 1/norm, one value per distinct
+  // stabiliser count, and the rows gather v itself: no pass over v, no u.  Unless
+  // that makes the entries six bytes (36 sites at k = 0: 2^4 values at most beside
+  // the columns) or the table large: the pass is 1 % of those sectors' H v, while
+  // on a small sector it is one launch of two (16 sites, with fewer queries a launch: 11.7 -> 7.5 us).
+  const int n_stab = std::max(1, __builtin_popcountll(S.lids));
+  const int64_t n_fold = (int64_t)S.n_vals * n_stab;
+  S.folded = n_fold <= 4096 && (pack_bits(n_fold) || !pack_bits(S.n_vals));
+  S.n_rvals = S.folded ? (int)n_fold : S.n_vals;
+  P.n_stab = S.folded ? n_stab : 1;
+  std::memset(P.stab_idx, 0, sizeof P.stab_idx);
   const char* fmt_env = std::getenv("EDG_ROW_FORMAT");
   const bool want_split = fmt_env && std::strcmp(fmt_env, "split") == 0;
-  const int cb = 32 - vb;
-  S.pack_cb = (!want_split && vb < 32 && P.n_p < (int64_t(1) << cb)) ? cb : 0;
+  S.pack_cb = want_split ? 0 : pack_bits(S.n_rvals);
   const double entry_bytes = S.pack_cb ? 4.0 : 6.0;
+  size_t fold_bytes = 0;
+  if (S.folded) {
+    std::vector<uint8_t> both(24 * n_fold);
+    double2* r64 = reinterpret_cast<double2*>(both.data());
+    float2* r32 = reinterpret_cast<float2*>(both.data() + 16 * n_fold);
+    int at = 0;
+    for (int l = 1; l <= 64; ++l) {
+      if (!((S.lids >> (l - 1)) & 1ull)) continue;
+      P.stab_idx[l] = (uint8_t)at;
+      for (int v = 0; v < S.n_vals; ++v) {
+        const double2 x = make_double2(S.values_host[v].x * P.nrm_inv[l], S.values_host[v].y * P.nrm_inv[l]);
+        r64[(size_t)v * n_stab + at] = x;
+        r32[(size_t)v * n_stab + at] = make_float2((float)x.x, (float)x.y);
+      }
+      ++at;
+    }
+    fold_bytes = both.size();
+    cudaError_t ce = cudaMalloc(&S.row_values, fold_bytes);
+    if (ce == cudaSuccess) ce = cudaMemcpy(S.row_values, both.data(), fold_bytes, cudaMemcpyHostToDevice);
+    if (ce != cudaSuccess) {
+      cudaGetLastError();
+      free_targets(S);
+      err = "stored targets: out of device memory for the value table";
+      return EDG_ERR_NOMEM;
+    }
+    S.rtab64 = static_cast<double2*>(S.row_values);
+    S.rtab32 = reinterpret_cast<float2*>(S.rtab64 + n_fold);
+  } else {
+    S.rtab64 = S.vtab64;
+    S.rtab32 = S.vtab32;
+  }
 
   cudaStream_t st = S.stream;
   const int64_t n = P.n_p;
   uint32_t* counts = nullptr;
   unsigned long long *sums = nullptr, *tot = nullptr;
   const int64_t n_chunks = (n + kChunk - 1) / kChunk;
-  cudaError_t e = cudaMalloc(&counts, sizeof(uint32_t) * n);
+  cudaError_t e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMalloc(&counts, sizeof(uint32_t) * n);
   if (e == cudaSuccess) e = cudaMalloc(&sums, sizeof(unsigned long long) * n_chunks);
   if (e == cudaSuccess) e = cudaMalloc(&tot, sizeof(unsigned long long));
   if (e == cudaSuccess) e = cudaMalloc(&S.row_ptr, sizeof(uint64_t) * (n + 1));
@@ -514,14 +567,14 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   }
   e = cudaMalloc(&S.col, sizeof(uint32_t) * std::max<unsigned long long>(1, nnz));
   if (e == cudaSuccess && !S.pack_cb) e = cudaMalloc(&S.vid, sizeof(uint16_t) * std::max<unsigned long long>(1, nnz));
-  if (e == cudaSuccess) e = cudaMalloc(&S.ubuf.ptr, (size_t)(16 * n));
+  if (e == cudaSuccess && !S.folded) e = cudaMalloc(&S.ubuf.ptr, (size_t)(16 * n));
   if (e != cudaSuccess) {
     cleanup();
     free_targets(S);
     err = "stored targets: out of device memory";
     return EDG_ERR_NOMEM;
   }
-  S.ubuf.bytes = (size_t)(16 * n);
+  S.ubuf.bytes = S.folded ? 0 : (size_t)(16 * n);
   if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, true>);
   else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, true>);
   else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, true>);
@@ -535,7 +588,7 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     return EDG_ERR_CUDA;
   }
   P.n_targets = (int64_t)nnz;
-  S.targets_bytes = (S.pack_cb ? 4 : 6) * nnz + 8 * (n + 1) + 8 * n + 16 * n;
+  S.targets_bytes = (S.pack_cb ? 4 : 6) * nnz + 8 * (n + 1) + 8 * n + S.ubuf.bytes + fold_bytes;
   S.device_bytes += S.targets_bytes;
   e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
   return e == cudaSuccess ? EDG_OK : EDG_ERR_CUDA;
@@ -653,6 +706,7 @@ cudaError_t launch_u_in(const Sector& S, const void* v_src, void* v_dst, bool fp
 }
 
 cudaError_t launch_hv_stored(const Sector& S, const void* v, void* w, bool fp64, cudaStream_t st) {
+  if (S.folded) return launch_hv_rows(S, v, v, w, fp64, 0, S.P.n_p, st);
   const cudaError_t e = launch_u(S, v, S.ubuf.ptr, fp64, st);
   return e == cudaSuccess ? launch_hv_rows(S, v, S.ubuf.ptr, w, fp64, 0, S.P.n_p, st) : e;
 }

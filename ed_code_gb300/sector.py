@@ -49,6 +49,7 @@ class GpuSector:
         else:
             N.check(N.lib().edg_sector_create(C.byref(m), self.n_ones, int(model.kx), int(model.ky), C.byref(h)))
         self._h = h
+        self._edg_hv = N.lib().edg_hv
         info = N.edg_sector_info()
         N.check(N.lib().edg_sector_get_info(self._h, C.byref(info)))
         self.info = {f: getattr(info, f) for f, _ in N.edg_sector_info._fields_}
@@ -139,15 +140,18 @@ class GpuSector:
         """w = H v on CUDA tensors (complex128 or complex64, n_p entries)."""
         import torch
 
-        if v.dtype not in (torch.complex128, torch.complex64) or w.dtype != v.dtype:
+        dt = v.dtype
+        code = N.EDG_C64 if dt is torch.complex64 else N.EDG_C128 if dt is torch.complex128 else -1
+        if code < 0 or w.dtype is not dt:
             raise TypeError("v and w must both be complex128 or both complex64")
         if not (v.is_cuda and w.is_cuda and v.is_contiguous() and w.is_contiguous()):
             raise ValueError("v and w must be contiguous CUDA tensors")
         if v.numel() != self.n_p or w.numel() != self.n_p:
             raise ValueError(f"v and w must have {self.n_p} entries")
-        code = N.EDG_C128 if v.dtype == torch.complex128 else N.EDG_C64
-        st = stream.cuda_stream if stream is not None else torch.cuda.current_stream().cuda_stream
-        N.check(N.lib().edg_hv(self._h, C.c_void_p(v.data_ptr()), C.c_void_p(w.data_ptr()), code, C.c_void_p(st)))
+        st = (torch.cuda.current_stream() if stream is None else stream).cuda_stream
+        rc = self._edg_hv(self._h, v.data_ptr(), w.data_ptr(), code, st)
+        if rc:
+            N.check(rc)
 
     def solve_plain(self, n_ev: int = 2, iterations: int = 100, ncycles: int = 10, tol: float = 1e-11,
                     seed: int = 0, dense_threshold: int = 10000, want_vectors: bool = False, log=None):
@@ -194,11 +198,12 @@ class GpuSector:
     def hv_block(self, v, w, stream=None) -> None:
         """W = H V for torch tensors of shape (n_p, 2) or (n_p, 4) (the vectors
         interleaved by row), on the device (edg_hv_block)."""
+        import torch
+
         nv = int(v.shape[1])
-        code = N.EDG_C128 if v.dtype == __import__("torch").complex128 else N.EDG_C64
+        code = N.EDG_C128 if v.dtype == torch.complex128 else N.EDG_C64
         st = stream.cuda_stream if stream is not None else 0
-        N.check(N.lib().edg_hv_block(self._h, C.c_void_p(v.data_ptr()), C.c_void_p(w.data_ptr()), nv, code,
-                                     C.c_void_p(st)))
+        N.check(N.lib().edg_hv_block(self._h, v.data_ptr(), w.data_ptr(), nv, code, st))
 
     def count_offdiag(self) -> int:
         n = C.c_int64()

@@ -99,3 +99,32 @@ def test_matrix_free_of_every_search_matches_oracle(cuda_device, Lx, Ly, Sz, k, 
             assert sec.build_targets()
         for dt, tol in ((np.complex128, 1e-13), (np.complex64, 2e-5)):
             assert np.abs(sec.sHv(v.astype(dt), dtype=dt) - w).max() / scale <= tol, (stored, dt)
+
+
+@pytest.mark.parametrize("nv", [2, 4])
+def test_block_hv_takes_vectors_between_16_byte_boundaries(cuda_device, nv):
+    """FP32 vectors that start 8 bytes past a 16-byte boundary: the same bits as
+    aligned ones (the rows' gathers are 16-byte loads), and as one vector alone
+    that starts there."""
+    import torch
+
+    from ed_code_gb300 import lattice as L
+    from ed_code_gb300 import sector
+
+    sec = sector.GpuSector(L.make_model(L.TorusSpec("triangular", 5, 4, Jz=0.7, Ch=0.3), 0, 1, 2, bowties=False))
+    assert sec.build_targets()
+    V = torch.randn((sec.n_p, nv), dtype=torch.complex64, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    W = torch.empty_like(V)
+    sec.hv_block(V, W)
+    flat, out = (torch.zeros(sec.n_p * nv + 1, dtype=torch.complex64, device="cuda") for _ in range(2))
+    odd, wodd = flat[1:].view(sec.n_p, nv), out[1:].view(sec.n_p, nv)
+    odd.copy_(V)
+    assert odd.data_ptr() % 16 == 8
+    sec.hv_block(odd, wodd)
+    torch.cuda.synchronize()
+    assert torch.equal(W, wodd)
+    one, w1 = flat[1: sec.n_p + 1], out[1: sec.n_p + 1]
+    one.copy_(V[:, 0])
+    sec.hv(one, w1)
+    torch.cuda.synchronize()
+    assert torch.equal(w1, W[:, 0].contiguous())
