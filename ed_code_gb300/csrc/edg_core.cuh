@@ -364,7 +364,7 @@ struct PackedRows {
   }
   static __device__ __forceinline__ bool single(Bytes hit) { return (hit & (hit - 1)) == 0; }
   static __device__ __forceinline__ int row_of(Bytes hit) {  // lowest row in hit
-    return (sizeof(Bytes) == 8 ? __ffsll((long long)hit) : __ffs((int)hit)) / 8 - 1;
+    return (int)((unsigned)(sizeof(Bytes) == 8 ? __ffsll((long long)hit) : __ffs((int)hit)) >> 3) - 1;
   }
   static __device__ __forceinline__ Orbit search(State t, Bytes hit, const SectorParams& P, const uint16_t* rots) {
     const int Lx = P.L1, Ly = P.L2, N = P.n_sites;
@@ -380,7 +380,8 @@ struct PackedRows {
       while (rs) {
         const int a = __ffs((int)rs) - 1;
         rs &= rs - 1;
-        const State v = a == 0 ? u : ((u << a) & (State)P.rot_hi[a]) | ((u >> (Lx - a)) & (State)P.rot_lo[a]);
+        const State lo = (State)P.rot_lo[a];
+        const State v = ((u << a) & ~lo & full) | ((u >> (Lx - a)) & lo);
         if (v < best || stab == 0) {
           best = v;
           g = a + Lx * b;

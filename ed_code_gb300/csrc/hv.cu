@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kHvThreads, 4) k_hv(SectorView V, const typena
 // on rows that take the same turns, the gathers of several targets are in
 // flight together, and a target costs four FP64 multiply-adds (two when real)
 // instead of 16 FP64 instructions for its coefficient, phase, norm and product,
-// which was what bound it (FP64 pipe 83 % busy): 2,484 us -> 1,097 us at 28 sites in
+// which was what bound it (FP64 pipe 83 % busy): 2,484 us -> 1,037 us at 28 sites in
 // FP64.  The gathered entries would need v / norm; with trivial stabilisers the
 // norms are one factor of the row, and the few targets with others are added
 // apart.
@@ -248,14 +248,13 @@ __global__ void __launch_bounds__(kFreeThreads) k_hv_free(SectorView V, const ty
       const PassGroup& gr = H.groups[g];
       const St pm = (St)gr.mask, both = s & pm;
       const bool anti = both != 0 && both != pm;
-      if (!__any_sync(0xffffffffu, anti)) continue;
       if (anti) {
         facs += gr.facadd;
         bool known;
         const Orbit o = target_orbit<kOrb, false>((St)(s ^ pm), gr, row, P, H, V.n_chunks, known);
-        const int64_t j = position(o, V, P);
+        const int64_t j = kOrb >= kOrbPacked ? position_of(o.rep, V, P) : position(o, V, P);
         if (j >= 0) {
-          const uint32_t id = value_id(s, gr, o.g, V, P, H);
+          const uint32_t id = value_id(s, gr, o.g, V, P);
           if (o.stab == 1) {
             qc[cnt][lane] = (uint32_t)j;
             qi[cnt][lane] = (uint16_t)id;

@@ -120,16 +120,11 @@ __device__ __forceinline__ Orbit search(uint64_t t, const SectorParams& P, const
   return orbit_walk(t, P, H.p1, H.p2, H.p3, n_chunks);
 }
 
-// Position j of the representative o.rep; j < 0 when it is not an allowed
-// state (the reference's rep_loc < 0).
-static __device__ __forceinline__ int64_t position(const Orbit& o, const SectorView& V, const SectorParams& P) {
-  // A translate of t is an n_sites-bit word; anything else means the search
-  // found no candidate, and is treated as "no allowed representative" rather
-  // than used as a table index.
-  if (o.rep & ~P.full_mask) return -1;
-  if ((unsigned)o.g >= 64u || (unsigned)o.stab > 64u) return -1;
+// Position j of a representative that a search found; j < 0 when it is not an
+// allowed state
+static __device__ __forceinline__ int64_t position_of(uint64_t rep, const SectorView& V, const SectorParams& P) {
   int bit;
-  const uint32_t q = vrec_of(o.rep, &bit);
+  const uint32_t q = vrec_of(rep, &bit);
   if ((int64_t)q >= P.n_vrecs) return -1;  // larger than every representative
   const uint4 raw = __ldg(reinterpret_cast<const uint4*>(V.vrecs) + q);
   RankRec rec;
@@ -138,6 +133,17 @@ static __device__ __forceinline__ int64_t position(const Orbit& o, const SectorV
   rec.bits[1] = raw.z;
   rec.bits[2] = raw.w;
   return rank_lookup_bit(bit, rec);
+}
+
+// Position j of the representative o.rep; j < 0 when it is not an allowed
+// state (the reference's rep_loc < 0).
+static __device__ __forceinline__ int64_t position(const Orbit& o, const SectorView& V, const SectorParams& P) {
+  // A translate of t is an n_sites-bit word; anything else means the search
+  // found no candidate, and is treated as "no allowed representative" rather
+  // than used as a table index.
+  if (o.rep & ~P.full_mask) return -1;
+  if ((unsigned)o.g >= 64u || (unsigned)o.stab > 64u) return -1;
+  return position_of(o.rep, V, P);
 }
 
 template <typename Real, bool kTorus>

@@ -10,6 +10,7 @@ namespace edg {
 namespace {
 
 constexpr int kMaxRowSlots = 256;  // a row has at most one target per flip group
+constexpr int kMaxChPerGroup = 4;
 
 // A flip group as the kernels stage it: what a row needs to find out
 // whether the pair is anti-aligned, and where its sites sit on a packed torus.
@@ -18,9 +19,10 @@ struct PassGroup {
   uint64_t facadd;        // 1 << 16 * fid: counts the row's anti-aligned pairs by diagonal part
   double fac;
   uint16_t off;           // first value variant
-  int16_t a, ch_begin, ch_end;
+  int8_t a, n_ch;
   int8_t sa, sb, ba, bb;  // packed torus: bit offset of each site's row in the state, of its byte
-  int8_t top, pad[3];     // packed torus: the pair touches the top row
+  int8_t top;             // packed torus: the pair touches the top row
+  int8_t z[kMaxChPerGroup], pad[3];  // chirality sites
 };
 
 // Which orbit search the kernels use: the reference's walk, the row-rotation
@@ -47,14 +49,13 @@ int orb_of(const SectorParams& P) {
 
 struct PassSmem {
   PassGroup* groups;
-  int8_t* z;  // chirality sites
   const uint8_t* nk;
   const uint16_t* rots;
   const uint64_t *p1, *p2, *p3;
 };
 
 size_t pass_smem_bytes(const SectorParams& P, int orb, int row_bits, int n_chunks, int n_perm) {
-  size_t b = align16(sizeof(PassGroup) * P.n_groups) + align16(P.n_ch);
+  size_t b = align16(sizeof(PassGroup) * P.n_groups);
   if (orb == kOrbWalk) return b + (size_t)n_perm * n_chunks * 256 * sizeof(uint64_t);
   return b + align16((size_t)3 << row_bits);
 }
@@ -65,8 +66,6 @@ __device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, uint8
   size_t off = 0;
   H.groups = reinterpret_cast<PassGroup*>(sm);
   off += align16(sizeof(PassGroup) * P.n_groups);
-  H.z = reinterpret_cast<int8_t*>(sm + off);
-  off += align16(P.n_ch);
   for (int at = threadIdx.x; at < P.n_groups; at += blockDim.x) {
     const int g = V.order[at];
     const TermGroup src = V.groups[g];
@@ -75,9 +74,9 @@ __device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, uint8
     d.facadd = P.n_facs <= kMaxFacs ? 1ull << (16 * src.fid) : 0;
     d.fac = src.fac;
     d.off = V.voff[g];
-    d.a = (int16_t)src.a;
-    d.ch_begin = (int16_t)src.ch_begin;
-    d.ch_end = (int16_t)src.ch_end;
+    d.a = (int8_t)src.a;
+    d.n_ch = (int8_t)(src.ch_end - src.ch_begin);
+    for (int m = src.ch_begin, b = 0; m < src.ch_end && b < kMaxChPerGroup; ++m, ++b) d.z[b] = (int8_t)V.ch[m].z;
     if (kOrb >= kOrbPacked) {
       const int ya = src.a / P.L1, yb = src.b / P.L1;
       d.sa = (int8_t)(P.L1 * ya);
@@ -88,7 +87,6 @@ __device__ PassSmem stage_pass(const SectorView& V, const SectorParams& P, uint8
     }
     H.groups[at] = d;
   }
-  for (int m = threadIdx.x; m < P.n_ch; m += blockDim.x) H.z[m] = (int8_t)V.ch[m].z;
   if (kOrb == kOrbWalk) {
     const int n = V.n_perm * V.n_chunks * 256;
     uint64_t* p = reinterpret_cast<uint64_t*>(sm + off);
@@ -167,13 +165,79 @@ __device__ __forceinline__ Orbit target_orbit(typename OrbRows<kOrb>::T::State t
   return orbit_walk(t, P, H.p1, H.p2, H.p3, n_chunks);
 }
 
+// Targets with a stabiliser, on a packed torus.  Such a target is left alone by
+// one of the translations of prime order (at most 8 up to those that generate
+// the same subgroup; 8x4 has 3).  For a translation T and the pair's mask m,
+// T(s ^ m) = s ^ m just when s ^ T s = m ^ T m, a word of at most 4 bits: a row
+// whose s ^ T s has more bits than that under every T (all but 1 in 150 at 8x4)
+// has no such target, and all its targets are allowed, at every momentum.
+struct PrimeShifts {
+  int n;
+  int8_t x[8], y[8];
+};
+
+PrimeShifts prime_shifts(const SectorParams& P) {
+  PrimeShifts R{};
+  for (int y = 0; y < P.L2; ++y)
+    for (int x = 0; x < P.L1; ++x) {
+      int order = 1;
+      while (order * x % P.L1 || order * y % P.L2) ++order;
+      bool first = order > 1;  // of prime order, and the first of its subgroup
+      for (int q = 2; q < order; ++q)
+        first = first && order % q && (q * y % P.L2) * P.L1 + q * x % P.L1 > y * P.L1 + x;
+      if (!first || R.n == 8) continue;
+      R.x[R.n] = (int8_t)x;
+      R.y[R.n++] = (int8_t)y;
+    }
+  return R;
+}
+
+template <typename St>
+__device__ __forceinline__ St shifted(St t, const PrimeShifts& G, int g, const SectorParams& P) {
+  const uint64_t u = torus_rotate_rows((uint64_t)t, P.L1 * G.y[g], P.n_sites, P.full_mask);
+  return (St)torus_rotate_within(u, G.x[g], P.L1, P);
+}
+
+// m ^ T m of every translation and group (moved[g * n_groups + group])
+template <typename St>
+__device__ __forceinline__ void stage_moved(const PrimeShifts& G, const SectorParams& P, const PassSmem& H, St* moved) {
+  for (int k = threadIdx.x; k < P.n_groups * G.n; k += blockDim.x) {
+    const St m = (St)H.groups[k % P.n_groups].mask;
+    moved[k] = m ^ shifted(m, G, k / P.n_groups, P);
+  }
+}
+
+// the translations that may leave a target of s alone, as bits
+template <typename St>
+__device__ __forceinline__ uint32_t risky_shifts(St s, const PrimeShifts& G, const SectorParams& P) {
+  uint32_t risk = 0;
+  for (int g = 0; g < G.n; ++g) risk |= popc64(s ^ shifted(s, G, g, P)) <= 4 ? 1u << g : 0u;
+  return risk;
+}
+
+// has the target of an anti-aligned group a stabiliser?
+template <typename St>
+__device__ __noinline__ bool symmetric_target(St s, int at, uint32_t risk, const PrimeShifts& G, const SectorParams& P,
+                                              const St* moved) {
+  for (; risk; risk &= risk - 1) {
+    const int g = __ffs((int)risk) - 1;
+    if (moved[g * P.n_groups + at] == (s ^ shifted(s, G, g, P))) return true;
+  }
+  return false;
+}
+
 // The value id of a target: bit a of the state and the bits z of the group's
 // chirality terms, and the phase class of the translation (value_tables).
 template <typename St>
 __device__ __forceinline__ uint32_t value_id(St s, const PassGroup& gr, int g, const SectorView& V,
-                                             const SectorParams& P, const PassSmem& H) {
+                                             const SectorParams& P) {
   int variant = (int)((s >> gr.a) & 1u);
-  for (int m = gr.ch_begin, b = 1; m < gr.ch_end; ++m, ++b) variant |= (int)((s >> H.z[m]) & 1u) << b;
+  const int n = gr.n_ch;
+  if (n == 2) {  // an inner bond of a torus of triangles: no loop
+    variant |= (int)((s >> gr.z[0]) & 1u) << 1 | (int)((s >> gr.z[1]) & 1u) << 2;
+  } else {
+    for (int b = 0; b < n; ++b) variant |= (int)((s >> gr.z[b]) & 1u) << (b + 1);
+  }
   return __ldg(V.remap + (gr.off + variant) * P.n_cls + P.g2cls[g]);
 }
 

@@ -43,33 +43,37 @@ namespace edg {
 namespace {
 
 constexpr int kPassThreads = 128;
-constexpr int kMaxChPerGroup = 4;
+constexpr int kPassTurns = 16;  // 48: 0.1 ms of 10.6 more
 
 // Pass 1 (count) and pass 2 (fill) share this walk over the rows' targets: a
 // thread owns a row and all of them go through the flip groups together, those
 // of high sites first (`order`).
 // Neighbouring rows are neighbouring representatives, equal in their high
 // sites: a group of high sites is anti-aligned in the whole warp or in none of
-// it (and is then skipped by the warp), its search takes the same turns in
+// it, its search takes the same turns in
 // every lane, and its rank records and remap entries come from neighbouring
-// addresses.  Counting needs no rank for a target that is alone in its orbit
-// search (one candidate translate): its stabiliser is trivial, so it is
-// allowed.  The fill pass writes each entry's value id as
-// remap[(pair variant) x class], the index into the deduplicated value table
-// (value_tables), packed above the column when cb > 0 (csr_row.cuh).
+// addresses.  Counting takes this walk only where k_tgt_count cannot; it needs
+// no rank for a target that is alone in its orbit search (one candidate
+// translate): its stabiliser is trivial, so it is allowed.  The fill pass writes
+// each entry's value id as remap[(pair variant) x class], the index into the
+// deduplicated value table (value_tables), packed above the column when cb > 0
+// (csr_row.cuh).
 //
-// Both passes are bound by integer issue (ALU pipe 65 %, 17-20 lanes of a warp
-// active), not by memory.  With a warp per row and a lane per pair they took
-// 18.7 + 22.8 ms on the 18.8-million-state 8x4 triangular sector; this form
-// took 7.9 + 14.1 ms with 64-bit states, and the sector up to its first H v
-// 54 ms, 34 ms, and 29 ms with 32-bit states.
+// The pass is bound by integer issue (ALU pipe 77 %, 22 lanes of a warp active),
+// not by memory.  With a warp per row and a lane per pair it took 22.8 ms on the
+// 18.8-million-state 8x4 triangular sector; a lane per row on 32-bit states took
+// 12.4 ms, kPassTurns times the resident CTAs instead of one turn of them 10.1 ms
+// (rows differ in their searches, and the last CTAs ran alone for a third of the
+// time), and group fields read where they stand, without loops over the two
+// chirality sites or checks that a search on rows cannot fail, 9.6 ms.  Filling
+// idle lanes was slower (10.7 ms): queues in shared memory for the targets that
+// are their own representatives and for the others, so that each was taken by 32
+// lanes at a time, cost more instructions than the idle lanes.
 template <int kOrb, bool kFill>
-__global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb, uint32_t* __restrict__ counts,
-                                                           double* __restrict__ ezz,
-                                                           const uint64_t* __restrict__ row_ptr,
+__global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb, int slots_at,
+                                                           double* __restrict__ ezz, uint64_t* row_ptr,
                                                            uint32_t* __restrict__ col, uint16_t* __restrict__ vid) {
   __shared__ SectorParams P;
-  __shared__ uint2 slots[kFill ? kPassThreads / 32 : 1][kFill ? kMaxRowSlots : 1];
   extern __shared__ __align__(16) uint8_t sm[];
   for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
     reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
@@ -85,10 +89,12 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb,
     const St s = live ? (St)V.reps[i] : 0;  // no pair is anti-aligned past the end
     uint64_t facs = 0, pos = 0;
     uint32_t cnt = 0;
-    uint2* slot = slots[kFill ? threadIdx.x >> 5 : 0];
+    uint32_t len = 0;
+    uint2* slot = reinterpret_cast<uint2*>(sm + slots_at) + (threadIdx.x >> 5) * ng;
     if (kFill) {
       // where the slice's slots start, and which rows have them (csr_row.cuh)
       const Slice sl = slice_at(row_ptr, i, n_p);
+      len = (uint32_t)sl.len;
       uint32_t at = 0;
       __syncwarp();
       for (int k = 0; k < sl.mx; ++k) {
@@ -105,7 +111,6 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb,
       const PassGroup& gr = H.groups[g];
       const St pm = (St)gr.mask, both = s & pm;
       const bool anti = both != 0 && both != pm;
-      if (!__any_sync(0xffffffffu, anti)) continue;
       if (!anti) continue;
       if (!kFill) facs += gr.facadd;
       bool known;
@@ -114,9 +119,9 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb,
         if (known || position(o, V, P) >= 0) ++cnt;
         continue;
       }
-      const int64_t j = position(o, V, P);
+      const int64_t j = kOrb >= kOrbPacked ? position_of(o.rep, V, P) : position(o, V, P);
       if (j < 0) continue;
-      const uint32_t id = value_id(s, gr, o.g, V, P, H) * P.n_stab + P.stab_idx[o.stab];
+      const uint32_t id = value_id(s, gr, o.g, V, P) * P.n_stab + P.stab_idx[o.stab];
       const uint2 sk = slot[cnt++];
       const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
       if (cb) {
@@ -126,14 +131,83 @@ __global__ void __launch_bounds__(kPassThreads) k_tgt_pass(SectorView V, int cb,
         vid[p] = (uint16_t)id;
       }
     }
+    if (kFill)  // a slot left over would be a hole that the rows gather through
+      for (; cnt < len; ++cnt) {
+        const uint2 sk = slot[cnt];
+        const uint64_t p = pos + sk.x + __popc(sk.y & ((1u << (threadIdx.x & 31)) - 1u));
+        col[p] = (uint32_t)i;
+        if (!cb) vid[p] = 0;
+      }
     if (!kFill && live) {
-      counts[i] = cnt;
+      row_ptr[i] = cnt;
       ezz[i] = row_ezz(s, facs, P, H);
     }
   }
 }
 
-// 64-bit exclusive scan of the counts into row_ptr[0..n] (row_ptr[n] = total)
+// The count on a packed torus.  A target without a stabiliser is allowed, so a
+// row's entries are its anti-aligned pairs, less the few targets of risky rows
+// (row_walk.cuh) that have one and no allowed representative.  That takes six
+// instructions a pair where a search for every target took about 90 (5.7 ms for
+// the 18.8 million rows of the 8x4 triangular sector, bound by integer issue);
+// here 0.68 ms.
+template <typename St>
+struct __align__(16) CountGroup {
+  uint64_t facadd;
+  St mask;
+};
+
+// Has the target of an anti-aligned group no allowed representative?
+template <typename St>
+__device__ __noinline__ bool refused_target(St s, int at, uint32_t risk, const PrimeShifts& G, const SectorView& V,
+                                            const SectorParams& P, const PassSmem& H, const St* moved) {
+  return symmetric_target(s, at, risk, G, P, moved) &&
+         position(orbit_torus(s ^ (St)H.groups[at].mask, P, H.nk, H.rots), V, P) < 0;
+}
+
+template <int kOrb>
+__global__ void __launch_bounds__(kPassThreads) k_tgt_count(SectorView V, PrimeShifts shifts, int moved_at,
+                                                            double* __restrict__ ezz, uint64_t* __restrict__ counts) {
+  using St = typename OrbRows<kOrb>::T::State;
+  __shared__ SectorParams P;
+  __shared__ PrimeShifts G;
+  extern __shared__ __align__(16) uint8_t sm[];
+  for (int i = threadIdx.x; i < (int)(sizeof(SectorParams) / 8); i += blockDim.x)
+    reinterpret_cast<uint64_t*>(&P)[i] = reinterpret_cast<const uint64_t*>(V.params)[i];
+  if (threadIdx.x == 0) G = shifts;
+  __syncthreads();
+  const PassSmem H = stage_pass<kOrb>(V, P, sm);
+  __syncthreads();
+  const int ng = P.n_groups;
+  CountGroup<St>* groups = reinterpret_cast<CountGroup<St>*>(sm + moved_at);
+  St* moved = reinterpret_cast<St*>(groups + ng);
+  for (int at = threadIdx.x; at < ng; at += blockDim.x) groups[at] = {H.groups[at].facadd, (St)H.groups[at].mask};
+  stage_moved(G, P, H, moved);
+  __syncthreads();
+  const int64_t n_p = P.n_p, stride = (int64_t)gridDim.x * blockDim.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_p; i += stride) {
+    const St s = (St)V.reps[i];
+    uint64_t facs = 0;
+    uint32_t cnt = 0;
+#pragma unroll 4
+    for (int g = 0; g < ng; ++g) {
+      const St pm = groups[g].mask, both = s & pm;
+      if (both != 0 && both != pm) {
+        ++cnt;
+        facs += groups[g].facadd;
+      }
+    }
+    if (const uint32_t risk = risky_shifts(s, G, P))
+      for (int g = 0; g < ng; ++g) {
+        const St both = s & groups[g].mask;
+        if (both != 0 && both != groups[g].mask && refused_target(s, g, risk, G, V, P, H, moved)) --cnt;
+      }
+    counts[i] = cnt;
+    ezz[i] = row_ezz(s, facs, P, H);
+  }
+}
+
+// 64-bit exclusive scan of the counts in row_ptr[0..n-1], in place (row_ptr[n] = total)
 constexpr int kScan = 256, kScanPer = 16, kChunk = kScan * kScanPer;
 
 __device__ __forceinline__ unsigned long long block_scan64(unsigned long long x, unsigned long long* tot) {
@@ -164,7 +238,7 @@ __device__ __forceinline__ unsigned long long block_scan64(unsigned long long x,
   return r;
 }
 
-__global__ void __launch_bounds__(kScan) k_scan64_chunks(const uint32_t* __restrict__ in, int64_t n,
+__global__ void __launch_bounds__(kScan) k_scan64_chunks(const uint64_t* __restrict__ in, int64_t n,
                                                           unsigned long long* __restrict__ sums) {
   const int64_t b = (int64_t)blockIdx.x * kChunk + (int64_t)threadIdx.x * kScanPer;
   unsigned long long s = 0;
@@ -191,22 +265,22 @@ __global__ void __launch_bounds__(kScan) k_scan64_sums(unsigned long long* __res
   if (threadIdx.x == 0) *total = carry;
 }
 
-__global__ void __launch_bounds__(kScan) k_scan64_apply(const uint32_t* __restrict__ in, int64_t n,
+__global__ void __launch_bounds__(kScan) k_scan64_apply(uint64_t* io, int64_t n,
                                                          const unsigned long long* __restrict__ offs,
-                                                         const unsigned long long* __restrict__ total,
-                                                         uint64_t* __restrict__ out) {
+                                                         const unsigned long long* __restrict__ total) {
   const int64_t b = (int64_t)blockIdx.x * kChunk + (int64_t)threadIdx.x * kScanPer;
   unsigned long long s = 0;
   for (int k = 0; k < kScanPer; ++k)
-    if (b + k < n) s += in[b + k];
+    if (b + k < n) s += io[b + k];
   __shared__ unsigned long long tot;
   unsigned long long run = block_scan64(s, &tot) + offs[blockIdx.x];
   for (int k = 0; k < kScanPer; ++k)
     if (b + k < n) {
-      out[b + k] = run;
-      run += in[b + k];
+      const uint64_t x = io[b + k];
+      io[b + k] = run;
+      run += x;
     }
-  if (blockIdx.x == 0 && threadIdx.x == 0) out[n] = *total;
+  if (blockIdx.x == 0 && threadIdx.x == 0) io[n] = *total;
 }
 
 // u_j = v_j / norm_j
@@ -267,19 +341,18 @@ __global__ void k_u_scale_in(const typename CT2<Real>::T* __restrict__ v, const 
   }
 }
 
-// Grid of a grid-stride kernel: the CTAs that fit on every SM at once, at most
-// cap per SM when cap > 0, no more than the work needs.
+// Grid of a grid-stride kernel: `turns` times the CTAs that fit on every SM at
+// once, no more than the work needs.
 template <typename K>
-int grid_for(K kernel, size_t smem, int64_t work, int threads, int cap = 0) {
+int grid_for(K kernel, size_t smem, int64_t work, int threads, int turns) {
   int dev = 0, sms = 0, per_sm = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-  if (cap > 0 && per_sm > cap) per_sm = cap;
   if (per_sm < 1) per_sm = 1;
   const int64_t want = (work + threads - 1) / threads;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)sms * per_sm * turns));
 }
 
 // The row kernel's tuned choices as template arguments: entries of a row in
@@ -518,20 +591,14 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
 
   cudaStream_t st = S.stream;
   const int64_t n = P.n_p;
-  uint32_t* counts = nullptr;
   unsigned long long *sums = nullptr, *tot = nullptr;
   const int64_t n_chunks = (n + kChunk - 1) / kChunk;
   cudaError_t e = cudaMemcpy(S.dP, &P, sizeof(P), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMalloc(&counts, sizeof(uint32_t) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&sums, sizeof(unsigned long long) * n_chunks);
-  if (e == cudaSuccess) e = cudaMalloc(&tot, sizeof(unsigned long long));
+  if (e == cudaSuccess) e = cudaMalloc(&sums, sizeof(unsigned long long) * (n_chunks + 1));
+  if (e == cudaSuccess) tot = sums + n_chunks;
   if (e == cudaSuccess) e = cudaMalloc(&S.row_ptr, sizeof(uint64_t) * (n + 1));
   if (e == cudaSuccess) e = cudaMalloc(&S.ezz, sizeof(double) * n);
-  auto cleanup = [&]() {
-    cudaFree(counts);
-    cudaFree(sums);
-    cudaFree(tot);
-  };
+  auto cleanup = [&]() { cudaFree(sums); };
   if (e != cudaSuccess) {
     cleanup();
     free_targets(S);
@@ -539,19 +606,25 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     return EDG_ERR_NOMEM;
   }
   const int orb = orb_of(P);
-  const size_t smem = pass_smem_bytes(P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm);
-  auto pass = [&](auto kern) {
-    kern<<<grid_for(kern, smem, n, kPassThreads), kPassThreads, smem, st>>>(
-        S.V, S.pack_cb, counts, S.ezz, S.row_ptr, S.col, S.vid);
+  const size_t terms = align16(pass_smem_bytes(P, orb, S.V.row_bits, S.V.n_chunks, S.V.n_perm));
+  auto pass = [&](auto kern, size_t smem) {
+    kern<<<grid_for(kern, smem, n, kPassThreads, kPassTurns), kPassThreads, smem, st>>>(
+        S.V, S.pack_cb, (int)terms, S.ezz, S.row_ptr, S.col, S.vid);
   };
-  if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, false>);
-  else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, false>);
-  else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, false>);
-  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, false>);
-  else pass(k_tgt_pass<kOrbWalk, false>);
-  k_scan64_chunks<<<(unsigned)n_chunks, kScan, 0, st>>>(counts, n, sums);
+  const PrimeShifts G = prime_shifts(P);
+  auto count = [&](auto kern, size_t state) {
+    const size_t smem = terms + P.n_groups * (16 + 8 + state * G.n);
+    kern<<<grid_for(kern, smem, n, kPassThreads, kPassTurns), kPassThreads, smem, st>>>(S.V, G, (int)terms, S.ezz,
+                                                                                            S.row_ptr);
+  };
+  if (orb == kOrbPacked) count(k_tgt_count<kOrbPacked>, 4);
+  else if (orb == kOrbPacked32) count(k_tgt_count<kOrbPacked32>, 4);
+  else if (orb == kOrbPacked64) count(k_tgt_count<kOrbPacked64>, 8);
+  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, false>, terms);
+  else pass(k_tgt_pass<kOrbWalk, false>, terms);
+  k_scan64_chunks<<<(unsigned)n_chunks, kScan, 0, st>>>(S.row_ptr, n, sums);
   k_scan64_sums<<<1, kScan, 0, st>>>(sums, n_chunks, tot);
-  k_scan64_apply<<<(unsigned)n_chunks, kScan, 0, st>>>(counts, n, sums, tot, S.row_ptr);
+  k_scan64_apply<<<(unsigned)n_chunks, kScan, 0, st>>>(S.row_ptr, n, sums, tot);
   unsigned long long nnz = 0;
   e = cudaMemcpyAsync(&nnz, tot, sizeof(nnz), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -575,11 +648,12 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
     return EDG_ERR_NOMEM;
   }
   S.ubuf.bytes = S.folded ? 0 : (size_t)(16 * n);
-  if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, true>);
-  else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, true>);
-  else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, true>);
-  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, true>);
-  else pass(k_tgt_pass<kOrbWalk, true>);
+  const size_t fill = terms + kPassThreads / 32 * sizeof(uint2) * P.n_groups;
+  if (orb == kOrbPacked) pass(k_tgt_pass<kOrbPacked, true>, fill);
+  else if (orb == kOrbPacked32) pass(k_tgt_pass<kOrbPacked32, true>, fill);
+  else if (orb == kOrbPacked64) pass(k_tgt_pass<kOrbPacked64, true>, fill);
+  else if (orb == kOrbTorus) pass(k_tgt_pass<kOrbTorus, true>, fill);
+  else pass(k_tgt_pass<kOrbWalk, true>, fill);
   e = cudaStreamSynchronize(st);
   cleanup();
   if (e != cudaSuccess) {

@@ -128,3 +128,25 @@ def test_block_hv_takes_vectors_between_16_byte_boundaries(cuda_device, nv):
     sec.hv(one, w1)
     torch.cuda.synchronize()
     assert torch.equal(w1, W[:, 0].contiguous())
+
+
+@pytest.mark.parametrize("Lx,Ly,Sz,k", [
+    (4, 4, 0, (0, 0)), (4, 4, 0, (1, 0)), (4, 4, -2, (2, 2)),  # three halves of the torus
+    (6, 3, 0, (2, 0)), (3, 6, 0, (1, 3)),    # orders 2 and 3
+    (6, 5, -10, (0, 0)), (6, 5, -10, (3, 1)),  # orders 2, 3 and 5
+    (6, 6, -12, (0, 0)), (6, 6, -12, (3, 2)),    # seven shifts, 64-bit states
+    (8, 4, -8, (4, 2)), (4, 8, 0, (0, 4)),   # 32 sites, 4 and 8 rows
+])
+def test_rows_counted_without_a_search_are_complete(cuda_device, Lx, Ly, Sz, k):
+    """On a packed torus the rows' lengths come from the anti-aligned pairs and
+    the targets with a stabiliser, whose momentum may refuse them: against the
+    general search's count, and the rows against the matrix-free H*v (1e-13)."""
+    from ed_code_gb300 import lattice as L
+    from ed_code_gb300 import sector
+
+    sec = sector.GpuSector(L.make_model(L.TorusSpec("triangular", Lx, Ly, Jz=0.7, Ch=0.3), Sz, *k, bowties=False))
+    v = O.splitmix_vector(sec.n_p, 9)
+    w, n = sec.sHv(v), sec.count_offdiag()
+    assert sec.build_targets()
+    assert sec.info["n_targets"] == n
+    assert np.abs(sec.sHv(v) - w).max() / max(1.0, np.abs(w).max()) <= 1e-13
