@@ -53,6 +53,7 @@
 #include <cstdlib>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/edgpu.h"
@@ -705,13 +706,13 @@ struct Segment {
   SegDev d{};
   SegState st{};
   int64_t bytes = 0;
+  void* slab = nullptr;    // the segment's own arrays (SegDev V .. omega), one allocation
   bool cancelled = false;  // edg_batch_cancel: released at the next settle, no result values
 };
 
 void release(Segment& g) {
-  void* p[] = {g.d.V, g.d.w, g.d.u, g.d.alpha, g.d.beta, g.d.q, g.d.ywork, g.d.aux, g.d.omega};
-  for (void* x : p)
-    if (x) cudaFree(x);
+  cudaFree(g.slab);
+  g.slab = nullptr;
   g.d = SegDev{};
 }
 
@@ -873,8 +874,10 @@ int64_t seg_tile_rows(int tile_rows, int64_t n) {
   return (rows + 31) / 32 * 32;
 }
 
+constexpr int64_t kSlabAlign = 256;
 int64_t segment_bytes(int64_t n, int m, int want) {
-  return (int64_t)sizeof(float2) * n * (m + 3) + (int64_t)sizeof(double) * (6 * (m + 2) + 6 * (int64_t)want * m);
+  return (int64_t)sizeof(float2) * n * (m + 3) + (int64_t)sizeof(double) * (6 * (m + 2) + 6 * (int64_t)want * m) +
+         9 * kSlabAlign;
 }
 
 // copy the device step counters and statuses into the host mirror
@@ -1269,15 +1272,29 @@ int edg_batch_add(edg_batch* bh, edg_sector* sec, const edg_batch_request* req) 
   d.want = std::min(req->n_ev, m);
   d.check_every = B.opts.check_every;
   d.tol = req->tol;
-  cudaError_t e = cudaMalloc(&d.V, sizeof(float2) * n * (m + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d.w, sizeof(float2) * n);
-  if (e == cudaSuccess && !S.folded) e = cudaMalloc(&d.u, sizeof(float2) * n);
-  if (e == cudaSuccess) e = cudaMalloc(&d.alpha, sizeof(double) * (m + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d.beta, sizeof(double) * (m + 2));
-  if (e == cudaSuccess) e = cudaMalloc(&d.q, sizeof(double) * 2 * (m + 1));
-  if (e == cudaSuccess) e = cudaMalloc(&d.ywork, sizeof(double) * 6 * (size_t)d.want * m);
-  if (e == cudaSuccess) e = cudaMalloc(&d.aux, sizeof(double) * 2);
-  if (e == cudaSuccess && B.opts.reorth == 1) e = cudaMalloc(&d.omega, sizeof(double) * 2 * (m + 2));
+  // One allocation a segment: eight of them, and as many frees, were a twelfth of
+  // the time of a batch of small sectors (160 segments of 9,250 rows and 150
+  // steps: 106 -> 98 ms).
+  int64_t at = 0;
+  auto take = [&](auto*& p, int64_t count, bool on) {
+    if (g.slab && on) p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(static_cast<char*>(g.slab) + at);
+    if (on) at += ((int64_t)sizeof(*p) * count + kSlabAlign - 1) / kSlabAlign * kSlabAlign;
+  };
+  auto lay_out = [&]() {
+    at = 0;
+    take(d.V, n * (m + 1), true);
+    take(d.w, n, true);
+    take(d.u, n, !S.folded);
+    take(d.alpha, m + 1, true);
+    take(d.beta, m + 2, true);
+    take(d.q, 2 * (m + 1), true);
+    take(d.ywork, 6 * (int64_t)d.want * m, true);
+    take(d.aux, 2, true);
+    take(d.omega, 2 * (m + 2), B.opts.reorth == 1);
+  };
+  lay_out();
+  cudaError_t e = cudaMalloc(&g.slab, (size_t)at);
+  if (e == cudaSuccess) lay_out();
   if (e != cudaSuccess) {
     cudaGetLastError();
     release(g);
