@@ -533,9 +533,9 @@ def run_device(args, world, rank, local_rank):
         "cpu_baseline": cpu,
         "e2e": e2e,
         "clocks": clocks,
-        # per step: the u = v/norm pass plus one row kernel; the matrix-free
-        # kernel is one launch
-        "gpu_launches": args.steps * (2 if mode == "stored-rows" else 1),
+        # per step: the row kernel, with the u = v/norm pass before it where the
+        # rows need one (36 sites at k = 0); the matrix-free kernel is one launch
+        "gpu_launches": args.steps * sec.hv_launches,
     }
     if rank == 0:
         print(json.dumps(out), flush=True)
@@ -845,7 +845,7 @@ def main():
                     help="record the DRAM bytes per launch of --kernel from this ncu CSV in profiles/traffic.json "
                          "under --tag, and exit")
     ap.add_argument("--tag", default=None, help="--ingest-ncu: the record's key (hv_<mode>_<workload>_<dtype>)")
-    ap.add_argument("--kernel", default="k_hv_csr", help="--ingest-ncu: kernel name substring")
+    ap.add_argument("--kernel", default="k_hv_rows", help="--ingest-ncu: kernel name substring")
     ap.add_argument("--scale", type=float, default=1.0,
                     help="--ingest-ncu: units of a full launch / units of the captured launch")
     ap.add_argument("--note", default="", help="--ingest-ncu: how the capture was made")

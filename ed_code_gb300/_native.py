@@ -135,6 +135,7 @@ SIGNATURES = {
                                      C.POINTER(C.c_int)]),
     "edg_sector_build_targets": (C.c_int, [C.c_void_p, C.c_int64]),
     "edg_sector_free_targets": (C.c_int, [C.c_void_p]),
+    "edg_sector_hv_launches": (C.c_int, [C.c_void_p]),
     "edg_sector_tune": (C.c_int, [C.c_void_p, C.c_int, C.POINTER(C.c_int), C.c_void_p]),
     "edg_solve_plain": (C.c_int, [C.c_void_p, C.POINTER(edg_solver_opts), C.c_void_p, C.c_int64,
                                   C.POINTER(C.c_int64), C.c_void_p, C.c_int64, C.POINTER(edg_solver_stats)]),

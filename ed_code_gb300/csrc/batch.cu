@@ -4,14 +4,15 @@
 //
 // Every segment is a sector with stored rows (targets.cu) and a request
 // (eigenvalues wanted, maximum steps, tolerance, seed).  Per segment the batch
-// keeps its FP32 Krylov vectors V_0..V_m, w, u = v/norm, its FP64 alpha/beta
+// keeps its FP32 Krylov vectors V_0..V_m, w, u = v/norm where its rows are not
+// folded (targets.cu; folded ones gather V_j itself), its FP64 alpha/beta
 // and its own step counter and status in device memory, so segments join and
 // leave independently: a segment added while others are half way starts at
 // step 0 with the next graph.  The rows of all live segments are cut into
 // tiles of `tile_rows` rows, and each kernel below runs one CTA per tile that
 // reads its segment's descriptor.  One step is nine kernels:
 //
-//   k_b_hv          u_j = V_j / norm was written by the previous step;
+//   k_b_hv          (u_j = V_j / norm, where used, was written by the previous step)
 //                   w = H V_j (lanes_per_row / 2 entries of a row in flight) and the
 //                   tile's partial of alpha_j = Re<V_j|w>
 //   k_b_step        w -= alpha_j V_j + beta_j V_{j-1} and the tile's |w|^2

@@ -486,7 +486,7 @@ int edg_sector_get_info(const edg_sector* s, edg_sector_info* info) {
   info->ctas_per_sm = s->s.col ? s->s.csr_cps : 0;
   info->pipelined = s->s.col ? s->s.csr_pipe : 0;
   info->entry_bytes = s->s.col ? (s->s.pack_cb ? 4 : 6) : 0;
-  info->n_values = s->s.col ? s->s.n_rvals : 0;
+  info->n_values = s->s.col ? s->s.n_vals : 0;
   return EDG_OK;
 }
 
@@ -683,6 +683,8 @@ int edg_sector_free_targets(edg_sector* s) {
   cudaMemcpy(s->s.dP, &s->s.P, sizeof(SectorParams), cudaMemcpyHostToDevice);
   return EDG_OK;
 }
+
+int edg_sector_hv_launches(const edg_sector* s) { return s && s->s.col && !s->s.folded ? 2 : 1; }
 
 int edg_sector_tune(edg_sector* s, int lanes_per_row, int* chosen, double* ms) {
   if (!s) return fail(EDG_ERR_INVALID, "NULL sector");

@@ -33,6 +33,8 @@ constexpr int kRowThreads = 256, kRowWarps = kRowThreads / 32;
 // values 926 -> 226 us; FP32 at 30 sites 593 -> 392 us (L1 66 % busy, 0.52
 // sectors a nonzero from L2), at 36 sites 60.5 -> 55.3 ms (DRAM: the
 // re-translated targets miss L2); four FP32 vectors at 32 sites 5.68 -> 4.03 ms.
+// Folded rows (targets.cu) took another 10 us off the first, 17 us off 30 sites
+// and 0.17 ms off the block: the pass over v and its launch.
 // 256 threads: 512 and 1,024 left fewer warps an SM (30 sites 445 us), and a
 // register cap that would fit more CTAs measured 408 us.
 template <typename Real, int NV, bool kSmemTab, int kPol, int kFmt, int kU, int kG, bool kPipe>

@@ -15,7 +15,8 @@
 // H*v is then a sparse matrix-vector product with a value dictionary, a warp
 // per slice of 32 rows (csr_row.cuh, hv_rows.cuh):
 //     w_i = norm_i * sum_t vtab[vid_t] * u[col_t] + Ezz_i * v_i,
-//     u_j = v_j / norm_j (a streaming pass before the row loop).
+//     u_j = v_j / norm_j (a streaming pass before the row loop), or, with folded
+// rows (build_targets), u = v and a vtab that includes 1 / norm_j.
 // This stores the Hamiltonian's structure (4 bytes per nonzero, 56 GB for the
 // 36-site Sz=0, k=0 sector) instead of searching orbits every H*v; the matrix-free
 // kernels (hv.cu) remain for sectors whose entries do not fit.  The reference

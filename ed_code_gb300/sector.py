@@ -210,6 +210,11 @@ class GpuSector:
         N.check(N.lib().edg_count_offdiag(self._h, C.byref(n)))
         return int(n.value)
 
+    @property
+    def hv_launches(self) -> int:
+        """Kernels that one hv() launches (edg_sector_hv_launches)."""
+        return N.lib().edg_sector_hv_launches(self._h)
+
     def algorithmic_bytes(self, elem_bytes: int, nnz_off: Optional[int] = None) -> int:
         """Bytes one H*v must move at minimum.  Matrix-free: per row the
         representative (8), the stabiliser byte (1), v_i and w_i; per
@@ -220,22 +225,24 @@ class GpuSector:
         if self.info.get("n_targets", 0):
             # stored rows: v_i, stabiliser byte, w_i; per nonzero its entry
             # (4 bytes packed, 6 split) and one u_j; row offsets and diagonal;
-            # the u pass
+            # the u pass where there is one
             nnz = self.info["n_targets"]
             entry = self.info.get("entry_bytes") or 6
-            return (self.n_p * (2 * S + 1) + nnz * (S + entry) + 8 * (self.n_p + 1) + 8 * self.n_p
-                    + self.n_p * (2 * S + 1))
+            u_pass = self.n_p * (2 * S + 1) if self.hv_launches == 2 else 0
+            return self.n_p * (2 * S + 1) + nnz * (S + entry) + 8 * (self.n_p + 1) + 8 * self.n_p + u_pass
         return self.n_p * (8 + 1 + 2 * S) + nnz_off * S
 
     def algorithmic_bytes_block(self, elem_bytes: int, nnz_off: Optional[int], nv: int) -> int:
         """Bytes one block H*v on nv vectors must move (stored rows): the
         entries, row offsets and diagonal once; per vector v_i, w_i, one u_j
-        per nonzero and the u pass; the stabiliser byte twice (u pass, row)."""
+        per nonzero and the u pass where there is one; the stabiliser byte
+        once a pass."""
         S = elem_bytes
         nnz = self.info.get("n_targets", 0)
         entry = self.info.get("entry_bytes") or 6
-        return (nnz * entry + 8 * (self.n_p + 1) + 8 * self.n_p + 2 * self.n_p
-                + nv * (self.n_p * 2 * S + nnz * S + self.n_p * 2 * S))
+        passes = self.hv_launches  # the u pass and the rows, or the rows alone
+        return (nnz * entry + 8 * (self.n_p + 1) + 8 * self.n_p + passes * self.n_p
+                + nv * (self.n_p * 2 * S * passes + nnz * S))
 
     def close(self) -> None:
         if getattr(self, "_h", None):

@@ -128,11 +128,16 @@ int edg_hv(edg_sector* s, const void* v, void* w, int dtype, void* stream);
  * these rows instead of searching orbits.  Fails with EDG_ERR_NOMEM (sector
  * unchanged, still matrix-free) when they need more than max_bytes (<= 0: no
  * limit) or than is free; EDG_ERR_UNSUPPORTED for ChCh terms or more than
- * 65536 distinct values.  H*v calls on one sector must not overlap: they
+ * 65536 distinct values.  H*v calls on one sector must not overlap: they may
  * share a scratch vector.  Counterpart in the reference: the optional
  * sparse-matrix sHv (H_v.cpp:3-19), which stores complex values per nonzero. */
 int edg_sector_build_targets(edg_sector* s, int64_t max_bytes);
 int edg_sector_free_targets(edg_sector* s);
+
+/* Kernels that one edg_hv launches: 2 when the stored rows gather u = v / norm,
+ * written by a pass over v first, else 1 (rows whose values include the
+ * target's 1 / norm, and the matrix-free kernel). */
+int edg_sector_hv_launches(const edg_sector* s);
 
 /* Entries of a row in flight (lanes_per_row / 2: 4, 8 or 16; the rows are
  * stored by slices of 32 and a lane sums a row, so the parameter keeps only its
@@ -164,7 +169,8 @@ int edg_hv_host(edg_sector* s, const void* v, void* w, int dtype);
  * holds the device's free memory, and loops where a cudaMalloc or cudaFree
  * would synchronise the device.  No counterpart in the reference (its sHv runs
  * on the host).  Needs stored rows (edg_sector_build_targets) and the sector's
- * device current.  The u = v/norm scratch is a fixed 16 MiB array in the
+ * device current.  The u = v/norm scratch (of sectors that need it; the limits
+ * and the ordering hold for all) is a fixed 16 MiB array in the
  * library's device image, held on every GPU that loads it until exit, so
  * n_p may be at most 1,048,576 (EDG_C128) or 2,097,152 (EDG_C64); larger
  * sectors return EDG_ERR_INVALID.  The first call on a device looks the
@@ -179,7 +185,8 @@ int edg_hv_noalloc(edg_sector* s, const void* v, void* w, int dtype, void* strea
  * `stream`.  Each row's stored entries are read once and each gathered line
  * serves all the vectors, so the bytes per vector fall with n_vectors; every
  * vector gets the bits edg_hv gives it alone.  Needs stored rows; keeps a
- * scratch of n_p * n_vectors entries on the sector.  No counterpart in the
+ * scratch of n_p * n_vectors entries on the sector where edg_hv launches two
+ * kernels, or for complex64 vectors that do not start on a 16-byte boundary.  No counterpart in the
  * reference (its sHv takes one vector, H_v.cpp:192); it serves block solvers
  * and the FP64 Rayleigh quotients of several Ritz vectors. */
 int edg_hv_block(edg_sector* s, const void* v, void* w, int n_vectors, int dtype, void* stream);
