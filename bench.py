@@ -534,7 +534,7 @@ def run_device(args, world, rank, local_rank):
         "e2e": e2e,
         "clocks": clocks,
         # per step: the row kernel, with the u = v/norm pass before it where the
-        # rows need one (36 sites at k = 0); the matrix-free kernel is one launch
+        # rows need one (targets.cu); the matrix-free kernel is one launch
         "gpu_launches": args.steps * sec.hv_launches,
     }
     if rank == 0:

@@ -356,7 +356,14 @@ cudaError_t launch_free(const Sector& S, int orb, const void* v, void* w, cudaSt
   // 1,024 chirality sites and 2,048 values
   const Resident r = resident((const void*)kern, kFreeThreads, smem, 128 * 1024);
   const int64_t want = (S.P.n_p * wps + kFreeThreads - 1) / kFreeThreads;
-  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)r.sms * r.per_sm));
+  // Up to 16 turns of the CTAs that fit at once: rows differ in their searches, and
+  // one turn ends in a tail (FP32 at 28, 30 and 36 sites 831 -> 774 us, 3.74 ->
+  // 3.16 ms, 270 -> 231 ms; FP64 at 36 sites 284 -> 262 ms).  A CTA keeps one and a
+  // half sets of rows on average, for staging the tables is a cost of its own (one set
+  // each: 24 sites 73 -> 78 us in FP32, 28 sites 1,037 -> 1,056 us in FP64).
+  const int64_t once = (int64_t)r.sms * r.per_sm;
+  const int64_t turns = std::max<int64_t>(1, std::min<int64_t>(16, 2 * want / (3 * once)));
+  const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(want, once * turns));
   const CT* tab = reinterpret_cast<const CT*>(sizeof(Real) == 8 ? (const void*)S.vtab64 : (const void*)S.vtab32);
   kern<<<grid, kFreeThreads, smem, st>>>(S.V, tab, S.n_vals, (int)at, wps, reinterpret_cast<const CT*>(v),
                                          reinterpret_cast<CT*>(w));

@@ -106,13 +106,21 @@ RowsView<Real> rows_of(const Sector& S, const void* u) {
 }
 
 // Grid of the row kernel: the CTAs that fit on every SM at once, at most cap
-// per SM when cap > 0, no more than the slices need.
-template <typename K>
+// per SM when cap > 0, no more than the slices need; without a cap, several
+// turns of them, as slices differ in their length and their gathers' misses and
+// one turn ends in a tail of few CTAs.  FP64 takes 8 turns with one or two
+// vectors (28 sites 520 -> 497 us, 30 sites 1,937 -> 1,854 us, 36 sites 122.7 ->
+// 112.7 ms); FP32, and FP64 with four (28 sites 1,196 -> 1,253 us with 8), as many, up to 8, as leave a warp 64 slices, for every turn
+// starts its loads anew (36 sites 54.8 -> 52.3 ms; 8 turns at 30 sites, with
+// 5 slices a warp, 374 -> 385 us).
+template <typename Real, int NV, typename K>
 int rows_grid(K kernel, size_t smem, int64_t slices, int per_cta, int cap) {
   Resident r = resident((const void*)kernel, kRowThreads, smem, 96 * 1024);
   if (cap > 0 && r.per_sm > cap) r.per_sm = cap;
   const int64_t want = (slices + per_cta - 1) / per_cta;
-  return (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)r.sms * r.per_sm));
+  const int64_t once = (int64_t)r.sms * r.per_sm;
+  const int64_t most = sizeof(Real) == 8 && NV <= 2 ? 8 : std::min<int64_t>(8, slices / (64 * once * per_cta));
+  return (int)std::max<int64_t>(1, std::min<int64_t>(want, once * (cap > 0 ? 1 : std::max<int64_t>(1, most))));
 }
 
 // rows [r0, r1) of w = H v from u = v / norm
@@ -124,7 +132,7 @@ cudaError_t launch_rows_k(const Sector& S, const void* v, const void* u, void* w
   const int wps = warps_per_slice(S.P.n_p);
   const size_t smem = kSmemTab ? sizeof(CT) * S.n_rvals : 0;
   auto kern = k_hv_rows<Real, NV, kSmemTab, kPol, kFmt, kU, kG, kPipe>;
-  const int grid = rows_grid(kern, smem, (r1 - r0 + 31) / 32, kRowWarps / wps, S.csr_cps);
+  const int grid = rows_grid<Real, NV>(kern, smem, (r1 - r0 + 31) / 32, kRowWarps / wps, S.csr_cps);
   kern<<<grid, kRowThreads, smem, st>>>(rows_of<Real>(S, u), S.n_rvals, S.ezz, S.lid,
                                         params_field(S, offsetof(SectorParams, nrm)), r0, r1, wps,
                                         reinterpret_cast<const CT*>(v), reinterpret_cast<CT*>(w));
