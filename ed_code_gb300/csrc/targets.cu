@@ -545,7 +545,7 @@ int build_targets(Sector& S, int64_t max_bytes, std::string& err) {
   };
   // Folded rows: the values include the target's 1/norm, one value per distinct
   // stabiliser count, and the rows gather v itself: no pass over v, no u.  Unless
-  // that makes the entries six bytes (36 sites at k = 0: 2^4 values at most beside
+  // that makes the entries six bytes (36 sites: 2^4 values at most beside
   // the columns) or the table large: the pass is 1 % of those sectors' H v, while
   // on a small sector it is one launch of two (16 sites, with fewer queries a launch: 11.7 -> 7.5 us).
   const int n_stab = std::max(1, __builtin_popcountll(S.lids));
