@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(kHvThreads, 4) k_hv(SectorView V, const typena
 // on rows that take the same turns, the gathers of several targets are in
 // flight together, and a target costs four FP64 multiply-adds (two when real)
 // instead of 16 FP64 instructions for its coefficient, phase, norm and product,
-// which was what bound it (FP64 pipe 83 % busy): 2,484 us -> 1,037 us at 28 sites in
+// which was what bound it (FP64 pipe 83 % busy): 2,484 us -> 1,026 us at 28 sites in
 // FP64.  The gathered entries would need v / norm; with trivial stabilisers the
 // norms are one factor of the row, and the few targets with others are added
 // apart.
